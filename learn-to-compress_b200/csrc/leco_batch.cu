@@ -2,15 +2,18 @@
 // uint32/uint64 and mixed LeCo/FOR/Delta/poly codecs, encoded and decoded by
 // one persistent launch per pass.
 //
-// Work queue: the batch's blocks are listed column by column as work items of
-// 256/G consecutive blocks, G being the column's threads per block (32, 64, 128
-// or 256): one block per item for G = 256, eight for G = 32 (one warp each).
-// Every CTA (256 threads) of a persistent grid takes the next item from an atomic
-// ticket and runs the per-block encoder or decoder instance for that column's
-// codec, value type, G and unroll depth in each of its 256/G groups.  Items
-// are handed out in order and every CTA of the grid is resident, so the
-// encoder's per-column look-back (byte offsets) only ever waits on blocks that
-// are already being processed.
+// Work queue: the batch's blocks are listed column by column as work items.  A decoder
+// item is 256/G consecutive blocks, G being the column's threads per block (32, 64, 128
+// or 256): one block per item for G = 256, eight for G = 32 (one warp each).  An encoder
+// item is 256/R consecutive blocks of R rows of 32 values (leco_rows.cuh: one thread per
+// row), or one block of 512 rows in a launch of its own.  Every CTA of a persistent grid
+// takes the next item from an atomic ticket and runs the encoder or decoder instance for
+// that column's codec and value type (decoder: G and unroll depth too).  Items are handed
+// out in order and every CTA of the grid is resident, so the encoder's per-column
+// look-back (byte offsets, one word per item) only ever waits on items that are already
+// being processed.  The reference's sequential fits are part of the encoder item
+// (rows_fit): as a pass of their own, one lane per block, they took 606 of the 945 us of an
+// encode + decode pass over 20 columns of 64K-4M values, against 0 now.
 //
 // The reference has no counterpart: its drivers loop over blocks of one column
 // (experiments/leco_int_fix_template.cpp:111-127, :145-153).  The per-column
@@ -24,126 +27,21 @@
 
 #include "leco_batch.cuh"
 
-namespace leco {
-
-// Sequential reference fits for every block of the columns that need them, one warp
-// per 32 consecutive blocks of the batch (lane j: block g0 + j, whatever its column):
-// each step the warp loads 32 consecutive values of each of its blocks (one row per
-// block, coalesced; u32 and u64 rows mix) into shared memory while the next step's
-// values are already in flight to registers, and lane j adds its block's values to
-// its running sums in order -- the reference's loop (lr.h:72-77; Y sums of
-// polynomial_regression_internals.hpp:129-137), as seq_fit_tiled_kernel does for one
-// column.  A full step's conversions and products are taken before its adds.  (One
-// thread per block with its own loads waited ~50 ns per value on each load.)
-__global__ void __launch_bounds__(128) batch_seq_fit_kernel(BatchArgs B) {
-  __shared__ uint64_t tile[4][32][33];
-  __shared__ const uint8_t *row_ptr[4][32];
-  __shared__ uint32_t row_len[4][32], row_s[4][32];
-  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const uint64_t g0 = ((uint64_t)blockIdx.x * 4 + w) * 32, gb = g0 + lane;
-  if (g0 >= B.total) return;
-  uint32_t len = 0, s = 8, bs = 1;
-  int codec = kLinear;
-  const uint8_t *vals = nullptr;
-  const double *polyX = nullptr;
-  double *model = nullptr;
-  if (gb < B.total) {
-    const uint32_t ci = find_column(B.prefix, B.ncols, gb);
-    const DevCol &c = B.cols[ci];
-    if (c.seq) {
-      const uint64_t b = gb - __ldg(B.prefix + ci);
-      len = (uint32_t)umin64(c.bs, c.n - b * c.bs);
-      s = (uint32_t)c.dtype;
-      bs = c.bs;
-      codec = c.codec;
-      vals = reinterpret_cast<const uint8_t *>(c.values) + b * c.bs * s;
-      polyX = c.polyX;
-      model = B.models + gb * 3;
-    }
-  }
-  row_ptr[w][lane] = vals;
-  row_len[w][lane] = len;
-  row_s[w][lane] = s;
-  const bool poly = codec == kPoly2;
-  const bool any_poly = __any_sync(0xffffffffu, poly && len);
-  const uint32_t maxlen = __reduce_max_sync(0xffffffffu, len);
-  uint64_t nxt[32];
-  auto fetch = [&](uint32_t t0) {
-    const uint32_t i = t0 + lane;
-#pragma unroll
-    for (int r = 0; r < 32; ++r) {
-      const uint32_t lr = row_len[w][r];
-      uint64_t v = 0;
-      if (i < lr) {
-        const uint8_t *vr = row_ptr[w][r];
-        v = row_s[w][r] == 8 ? __ldg(reinterpret_cast<const uint64_t *>(vr) + i)
-                             : (uint64_t)__ldg(reinterpret_cast<const uint32_t *>(vr) + i);
-      }
-      nxt[r] = v;
-    }
-  };
-  __syncwarp();
-  double s0 = 0, s1 = 0, s2 = 0;  // linear: sumy sumxy; poly: Y0 Y1 Y2
-  if (maxlen) fetch(0);
-  for (uint32_t t0 = 0; t0 < maxlen; t0 += 32) {
-#pragma unroll
-    for (int r = 0; r < 32; ++r) tile[w][r][lane] = nxt[r];
-    __syncwarp();
-    if (t0 + 32 < maxlen) fetch(t0 + 32);
-    const uint32_t cnt = len > t0 ? (len - t0 < 32 ? len - t0 : 32) : 0;
-    const double dt0 = u32_to_double_fp64(t0);
-    if (cnt == 32) {
-      double yv[32];
-#pragma unroll
-      for (int c = 0; c < 32; ++c) yv[c] = __ull2double_rn(tile[w][lane][c]);  // a u32 value converts the same way
-      if (!any_poly) {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          s0 = __dadd_rn(s0, yv[c]);
-          s1 = __dadd_rn(s1, __dmul_rn(__dadd_rn(dt0, (double)c), yv[c]));  // i = t0 + c exactly
-        }
-      } else {
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const double di = __dadd_rn(dt0, (double)c);
-          s0 = __dadd_rn(s0, yv[c]);  // the reference's 1.0 * y is y
-          s1 = __dadd_rn(s1, __dmul_rn(di, yv[c]));
-          s2 = __dadd_rn(s2, __dmul_rn(__dmul_rn(di, di), yv[c]));
-        }
-      }
-    } else {
-      for (uint32_t c = 0; c < cnt; ++c) {
-        const double di = __dadd_rn(dt0, __uint2double_rn(c)), yi = __ull2double_rn(tile[w][lane][c]);
-        s0 = __dadd_rn(s0, yi);
-        s1 = __dadd_rn(s1, __dmul_rn(di, yi));
-        if (poly) s2 = __dadd_rn(s2, __dmul_rn(__dmul_rn(di, di), yi));
-      }
-    }
-    __syncwarp();
-  }
-  if (!len) return;
-  if (poly) store_seq_model<kPoly2>(model, s0, s1, s2, len, bs, polyX);
-  else store_seq_model<kLinear>(model, s0, s1, s2, len, bs, polyX);
-}
-
-}  // namespace leco
-
 using namespace leco;
 
 struct leco_batch {
   std::vector<leco_column_desc> cols;
   std::vector<uint64_t> prefix;
   int fit_mode = LECO_FIT_REFERENCE;
-  bool any_seq = false;
   int device = 0;
   DevCol *d_cols = nullptr;
   uint64_t *d_prefix = nullptr;
-  uint64_t *d_items = nullptr;
-  uint64_t nitems = 0;
-  uint8_t *d_ws = nullptr;  // status [total] | ticket | models [total*3]
-  uint64_t ws_bytes = 0, status_bytes = 0, models_off = 0;
-  uint32_t enc_smem = 0;
-  int enc_grid = 0, dec_grid = 0;
+  uint64_t *d_items = nullptr, *d_enc_items = nullptr;
+  uint64_t nitems = 0, enc_n[2] = {0, 0};
+  uint8_t *d_ws = nullptr;  // status [encoder items] | tickets
+  uint64_t ws_bytes = 0, status_bytes = 0;
+  uint32_t enc_smem[2] = {0, 0};
+  int enc_grid[2] = {0, 0}, dec_grid = 0;
   uint32_t *err = nullptr;               // library error word on this device
   cudaStream_t capture_stream = nullptr;  // graphs are captured here (the caller's stream may be the legacy default stream)
   cudaGraphExec_t graph[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -167,12 +65,14 @@ BatchArgs args_of(const leco_batch *b, uint32_t *err) {
   B.cols = b->d_cols;
   B.prefix = b->d_prefix;
   B.items = b->d_items;
+  B.enc_items = b->d_enc_items;
+  B.enc_n[0] = b->enc_n[0];
+  B.enc_n[1] = b->enc_n[1];
   B.nitems = b->nitems;
   B.ncols = (uint32_t)b->cols.size();
   B.total = b->prefix.back();
   B.status = reinterpret_cast<uint64_t *>(b->d_ws);
   B.ticket = reinterpret_cast<unsigned long long *>(b->d_ws + b->status_bytes);
-  B.models = reinterpret_cast<double *>(b->d_ws + b->models_off);
   B.error = err;
   return B;
 }
@@ -191,7 +91,6 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
   b->prefix.resize(ncols + 1);
   std::vector<DevCol> dc(ncols);
   uint64_t total = 0;
-  uint32_t max_smem = 0;
   for (uint32_t i = 0; i < ncols; ++i) {
     const leco_column_desc &c = h_cols[i];
     if (c.codec < kLinear || c.codec > kPoly2 || (c.dtype != 4 && c.dtype != 8) || !c.block_size ||
@@ -206,7 +105,6 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
     d.dtype = c.dtype;
     d.bs = c.block_size;
     d.seq = needs_seq(c.codec, c.dtype, c.block_size, fit_mode);
-    b->any_seq |= d.seq != 0;
     d.n = c.n;
     d.values = c.d_values;
     d.out = c.d_out;
@@ -222,6 +120,7 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
     }
     d.group = c.group_threads ? c.group_threads : (c.block_size <= kWarpBlock ? 32u : 256u);
     d.unroll = c.unroll ? c.unroll : 2u;
+    d.rows = rows_threads(c.block_size);
     d.pad = 0;
     if ((d.group != 32 && d.group != 64 && d.group != 128 && d.group != 256) ||
         (d.unroll != 1 && d.unroll != 2 && d.unroll != 4)) {
@@ -229,15 +128,18 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
       return berr(LECO_ERR_ARG, "leco_batch_create: column " + std::to_string(i) +
                                     ": group_threads must be 0, 32, 64, 128 or 256 and unroll 0, 1, 2 or 4");
     }
-    d.slice = (enc_smem_bytes(c.block_size, (uint32_t)c.dtype) + 15) / 16 * 16;
-    const uint32_t item_smem = d.slice * (256 / d.group);
+    // (the limit of group_threads: a group's values, held once for each group of 256 threads)
+    const uint32_t slice = (enc_smem_bytes(c.block_size, (uint32_t)c.dtype) + 15) / 16 * 16;
+    const uint32_t item_smem = slice * (256 / d.group);
     if (item_smem > kBatchMaxSmem) {
       delete b;
       return berr(LECO_ERR_ARG, "leco_batch_create: column " + std::to_string(i) + ": " + std::to_string(256 / d.group) +
-                                    " groups of " + std::to_string(d.slice) + " bytes of shared memory exceed the " +
+                                    " groups of " + std::to_string(slice) + " bytes of shared memory exceed the " +
                                     std::to_string(kBatchMaxSmem) + " a CTA may use");
     }
-    max_smem = std::max(max_smem, item_smem);
+    const int which = d.rows == 512;
+    b->enc_smem[which] = std::max(b->enc_smem[which], rows_layout(which ? 512 : 256, d.rows, (uint32_t)c.dtype,
+                                                                  (uint32_t)rows_sums(c.codec)).total);
   }
   // work items: (column << 32) | first block, 256/G blocks per item
   std::vector<uint64_t> items;
@@ -246,16 +148,29 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
     const uint64_t step = 256 / dc[i].group;
     for (uint64_t blk = 0; blk < nb; blk += step) items.push_back(((uint64_t)i << 32) | blk);
   }
+  // encoder items: (column << 32) | item, items of 256 threads before those of 512
+  std::vector<uint64_t> enc_items;
+  for (int which = 0; which < 2; ++which) {
+    for (uint32_t i = 0; i < ncols; ++i) {
+      if ((dc[i].rows == 512) != (which == 1)) continue;
+      const uint64_t nb = leco_num_blocks(h_cols[i].n, h_cols[i].block_size), per = which ? 1 : 256 / dc[i].rows;
+      dc[i].item0 = enc_items.size();
+      for (uint64_t k = 0; k * per < nb; ++k) enc_items.push_back(((uint64_t)i << 32) | k);
+    }
+    b->enc_n[which] = enc_items.size() - (which ? b->enc_n[0] : 0);
+  }
   b->nitems = items.size();
   b->prefix[ncols] = total;
   if (total > 0xffffffffull) {
     delete b;
     return berr(LECO_ERR_ARG, "leco_batch_create: more than 2^32 blocks");
   }
-  b->status_bytes = (total * 8 + 255) / 256 * 256;
-  b->models_off = b->status_bytes + 256;
-  b->ws_bytes = b->models_off + (b->any_seq ? (total * 24 + 255) / 256 * 256 : 0);
-  b->enc_smem = max_smem;
+  b->status_bytes = (enc_items.size() * 8 + 255) / 256 * 256;
+  b->ws_bytes = b->status_bytes + 256;
+  // the per-column calls encode through the same workspace
+  for (uint32_t i = 0; i < ncols; ++i)
+    b->ws_bytes = std::max(b->ws_bytes, leco_encode_workspace_bytes(h_cols[i].codec, h_cols[i].dtype, h_cols[i].n,
+                                                                    h_cols[i].block_size, fit_mode));
   cudaError_t e = cudaMalloc(&b->d_cols, ncols * sizeof(DevCol));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_prefix, (ncols + 1) * sizeof(uint64_t));
   if (e == cudaSuccess) e = cudaMalloc(&b->d_ws, b->ws_bytes);
@@ -263,21 +178,30 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
   if (e == cudaSuccess) e = cudaMemcpy(b->d_prefix, b->prefix.data(), (ncols + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(&b->d_items, std::max<size_t>(1, items.size()) * sizeof(uint64_t));
   if (e == cudaSuccess) e = cudaMemcpy(b->d_items, items.data(), items.size() * sizeof(uint64_t), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMalloc(&b->d_enc_items, std::max<size_t>(1, enc_items.size()) * sizeof(uint64_t));
+  if (e == cudaSuccess)
+    e = cudaMemcpy(b->d_enc_items, enc_items.data(), enc_items.size() * sizeof(uint64_t), cudaMemcpyHostToDevice);
   if (e == cudaSuccess && leco::device_error_word(&b->err)) e = cudaErrorUnknown;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess && max_smem > 48 * 1024)
-    e = cudaFuncSetAttribute(batch_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
-  int sms = 148, per_enc = 1, per_dec = 1;
+  if (e == cudaSuccess && b->enc_smem[0] > 48 * 1024)
+    e = cudaFuncSetAttribute(batch_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->enc_smem[0]);
+  if (e == cudaSuccess && b->enc_smem[1] > 48 * 1024)
+    e = cudaFuncSetAttribute(batch_encode_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->enc_smem[1]);
+  int sms = 148, per_enc[2] = {1, 1}, per_dec = 1;
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_enc, batch_encode_kernel, 256, max_smem);
+  if (e == cudaSuccess && b->enc_n[0])
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_enc[0], batch_encode_kernel, 256, b->enc_smem[0]);
+  if (e == cudaSuccess && b->enc_n[1])
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_enc[1], batch_encode_large_kernel, 512, b->enc_smem[1]);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_dec, batch_decode_kernel, 256, 0);
-  if (e != cudaSuccess || per_enc < 1 || per_dec < 1) {
+  if (e != cudaSuccess || per_enc[0] < 1 || per_enc[1] < 1 || per_dec < 1) {
     leco_batch_destroy(b);
     return berr(e != cudaSuccess ? LECO_ERR_CUDA : LECO_ERR_ARG,
                 std::string("leco_batch_create: ") + (e != cudaSuccess ? cudaGetErrorString(e) : "no resident CTA fits"));
   }
   // every CTA of the persistent grid must be resident (the look-back waits on them)
-  b->enc_grid = (int)std::min<uint64_t>(b->nitems, (uint64_t)sms * per_enc);
+  for (int which = 0; which < 2; ++which)
+    b->enc_grid[which] = (int)std::min<uint64_t>(b->enc_n[which], (uint64_t)sms * per_enc[which]);
   b->dec_grid = (int)std::min<uint64_t>(b->nitems, (uint64_t)sms * per_dec);
   *out = b;
   return LECO_OK;
@@ -291,6 +215,7 @@ int leco_batch_destroy(leco_batch *b) {
   if (b->d_cols) cudaFree(b->d_cols);
   if (b->d_prefix) cudaFree(b->d_prefix);
   if (b->d_items) cudaFree(b->d_items);
+  if (b->d_enc_items) cudaFree(b->d_enc_items);
   if (b->d_ws) cudaFree(b->d_ws);
   delete b;
   return LECO_OK;
@@ -303,9 +228,8 @@ int leco_batch_encode(leco_batch *b, leco_stream_t stream) {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const BatchArgs B = args_of(b, b->err);
   cudaError_t e = cudaMemsetAsync(b->d_ws, 0, b->status_bytes + 256, st);  // look-back words + ticket
-  if (e == cudaSuccess && b->any_seq)
-    batch_seq_fit_kernel<<<(unsigned)((B.total + 127) / 128), 128, 0, st>>>(B);  // four warps of 32 blocks
-  if (e == cudaSuccess) batch_encode_kernel<<<b->enc_grid, 256, b->enc_smem, st>>>(B);
+  if (e == cudaSuccess && b->enc_grid[0]) batch_encode_kernel<<<b->enc_grid[0], 256, b->enc_smem[0], st>>>(B);
+  if (e == cudaSuccess && b->enc_grid[1]) batch_encode_large_kernel<<<b->enc_grid[1], 512, b->enc_smem[1], st>>>(B);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? LECO_OK : berr(LECO_ERR_CUDA, std::string("leco_batch_encode: ") + cudaGetErrorString(e));
 }

@@ -6,14 +6,16 @@
 
 #include "leco_decode.cuh"
 #include "leco_encode.cuh"
+#include "leco_rows.cuh"
 
 namespace leco {
 
 struct DevCol {
   int32_t codec, dtype;
   uint32_t bs, seq;
-  uint32_t group, unroll;  // threads per block (32, 64, 128, 256), unroll depth (1, 2, 4)
-  uint32_t slice, pad;     // encoder shared memory per group (bytes)
+  uint32_t group, unroll;  // decoder: threads per block (32, 64, 128, 256), unroll depth (1, 2, 4)
+  uint32_t rows, pad;      // encoder: threads per block (rows_threads)
+  uint64_t item0;          // encoder: the column's first look-back word
   uint64_t n;
   const void *values;
   void *out;
@@ -23,16 +25,6 @@ struct DevCol {
   leco_dir_entry *dir;
   double polyX[10];
 };
-
-__device__ __forceinline__ uint32_t find_column(const uint64_t *__restrict__ prefix, uint32_t ncols, uint64_t gb) {
-  uint32_t lo = 0, hi = ncols;  // largest c with prefix[c] <= gb
-  while (hi - lo > 1) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (__ldg(prefix + mid) <= gb) lo = mid;
-    else hi = mid;
-  }
-  return lo;
-}
 
 #define LECO_BATCH_DISPATCH(codec, dtype, FN, ...)                 \
   do {                                                             \
@@ -56,19 +48,21 @@ __device__ __forceinline__ uint32_t find_column(const uint64_t *__restrict__ pre
 struct BatchArgs {
   const DevCol *cols;
   const uint64_t *prefix;  // [ncols + 1] blocks before each column
-  const uint64_t *items;   // [nitems] (column << 32) | first block
+  const uint64_t *items;   // decoder: [nitems] (column << 32) | first block
+  const uint64_t *enc_items;  // encoder: (column << 32) | item of the column, 256-thread items first
+  uint64_t enc_n[2];       // items of 256 and of 512 threads
   uint32_t ncols;
   uint64_t nitems;
   uint64_t total;          // blocks in the batch
-  uint64_t *status;        // [total] look-back words (zeroed per encode pass)
-  unsigned long long *ticket;  // zeroed per pass
-  double *models;          // [total * 3] sequential-fit models
+  uint64_t *status;        // one look-back word per encoder item (zeroed per encode pass)
+  unsigned long long *ticket;  // [3] zeroed per pass: the decoder's, the encoder's two
   uint32_t *error;
 };
 
 // Persistent kernels (one ticket = one work item), defined in leco_batch_encode.cu
 // and leco_batch_decode.cu.
 __global__ void __launch_bounds__(256, 3) batch_encode_kernel(BatchArgs B);
+__global__ void __launch_bounds__(512, 1) batch_encode_large_kernel(BatchArgs B);
 __global__ void __launch_bounds__(256, 4) batch_decode_kernel(BatchArgs B);
 
 }  // namespace leco

@@ -1,75 +1,56 @@
 // leco_batch_encode.cu -- the batch engine's persistent encode kernel (see
-// leco_batch.cu for the work queue).  A translation unit of its own: its many
-// per-codec, per-group and per-unroll encoder instances compile in parallel with
-// the decoder's.
+// leco_batch.cu for the work queue).  A translation unit of its own: its per-codec
+// encoder instances compile in parallel with the decoder's.
 #include "leco_batch.cuh"
 
 namespace leco {
 
-template <typename T, int CODEC, int G, int U>
-__device__ __forceinline__ void batch_encode_one(const BatchArgs &B, const DevCol &c, uint32_t ci, uint64_t b,
+template <typename T, int CODEC>
+__device__ __forceinline__ void batch_encode_one(const BatchArgs &B, const DevCol &c, uint32_t ci, uint64_t item,
                                                  uint8_t *smem) {
   EncodeArgs a;
   a.values = c.values;
   a.n = c.n;
   a.bs = c.bs;
-  const uint64_t p0 = __ldg(B.prefix + ci);
-  a.nb = __ldg(B.prefix + ci + 1) - p0;
+  a.nb = __ldg(B.prefix + ci + 1) - __ldg(B.prefix + ci);
   a.payload = c.payload;
   a.payload_cap = c.payload_cap;
   a.offsets = c.offsets;
   a.dir = c.dir;
-  a.seq_models = c.seq ? B.models + p0 * 3 : nullptr;
+  a.seq_models = nullptr;
   for (int i = 0; i < 10; ++i) a.polyX[i] = c.polyX[i];
-  a.status = B.status + p0;
+  a.status = B.status + c.item0;
   a.ticket = nullptr;
   a.error = B.error;
-  a.rows_area = 0;  // the batch's per-group slices hold the values only
-  encode_block<T, CODEC, G, U>(a, b, smem);
-}
-// The unroll depth changes only the u64 LeCo encoder; other codecs take one instance.
-template <typename T, int CODEC, int G>
-__device__ __forceinline__ void batch_encode_u(const BatchArgs &B, const DevCol &c, uint32_t ci, uint64_t b, uint8_t *smem) {
-  if constexpr (CODEC == kLinear && sizeof(T) == 8 && G != 32) {
-    switch (c.unroll) {
-      case 1: batch_encode_one<T, CODEC, G, 1>(B, c, ci, b, smem); return;
-      case 4: batch_encode_one<T, CODEC, G, 4>(B, c, ci, b, smem); return;
-      default: batch_encode_one<T, CODEC, G, 2>(B, c, ci, b, smem); return;
-    }
-  } else {
-    batch_encode_one<T, CODEC, G, 2>(B, c, ci, b, smem);
-  }
-}
-template <typename T, int CODEC>
-__device__ __forceinline__ void batch_encode_any(const BatchArgs &B, const DevCol &c, uint32_t ci, uint64_t b, uint8_t *smem) {
-  switch (c.group) {
-    case 32: batch_encode_u<T, CODEC, 32>(B, c, ci, b, smem); return;
-    case 64: batch_encode_u<T, CODEC, 64>(B, c, ci, b, smem); return;
-    case 128: batch_encode_u<T, CODEC, 128>(B, c, ci, b, smem); return;
-    default: batch_encode_u<T, CODEC, 256>(B, c, ci, b, smem); return;
-  }
+  encode_rows_item<T, CODEC, 0, false>(a, item, c.rows, c.seq != 0, false, smem);
 }
 
-// Persistent encode: one ticket = one work item; group g of the CTA takes block
-// first + g of the item with its own slice of shared memory.
-__global__ void __launch_bounds__(256, 3) batch_encode_kernel(BatchArgs B) {
-  extern __shared__ __align__(16) uint8_t smem[];
+// Persistent encode: one ticket = one item of 256 / rows consecutive blocks of a column
+// (which = 1: 512 threads, one block of 8193..16384 values).
+template <int which>
+__device__ __forceinline__ void batch_encode_items(const BatchArgs &B, uint8_t *smem) {
   __shared__ unsigned long long item;
+  const uint64_t first = which ? B.enc_n[0] : 0, n = B.enc_n[which];
   for (;;) {
-    if (threadIdx.x == 0) item = atomicAdd(B.ticket, 1ull);
+    if (threadIdx.x == 0) item = atomicAdd(B.ticket + 1 + which, 1ull);
     __syncthreads();
     const uint64_t it = item;
     __syncthreads();
-    if (it >= B.nitems) break;
-    const uint64_t e = __ldg(B.items + it);
+    if (it >= n) break;
+    const uint64_t e = __ldg(B.enc_items + first + it);
     const uint32_t ci = (uint32_t)(e >> 32);
     const DevCol &c = B.cols[ci];
-    const uint32_t gi = threadIdx.x / c.group;
-    const uint64_t b = (e & 0xffffffffull) + gi;
-    if (b < __ldg(B.prefix + ci + 1) - __ldg(B.prefix + ci))
-      LECO_BATCH_DISPATCH(c.codec, c.dtype, batch_encode_any, B, c, ci, b, smem + (size_t)gi * c.slice);
+    LECO_BATCH_DISPATCH(c.codec, c.dtype, batch_encode_one, B, c, ci, e & 0xffffffffull, smem);
     __syncthreads();  // shared memory is reused by the next item
   }
+}
+__global__ void __launch_bounds__(256, 3) batch_encode_kernel(BatchArgs B) {
+  extern __shared__ __align__(256) uint8_t smem[];
+  batch_encode_items<0>(B, smem);
+}
+__global__ void __launch_bounds__(512, 1) batch_encode_large_kernel(BatchArgs B) {
+  extern __shared__ __align__(256) uint8_t smem[];
+  batch_encode_items<1>(B, smem);
 }
 
 }  // namespace leco

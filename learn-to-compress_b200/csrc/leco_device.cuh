@@ -367,30 +367,6 @@ __device__ __forceinline__ void group_reduce2(u128 &a, u128 &b, u128 *red) {
   }
 }
 
-// Reductions over warps 1.. of a CTA while warp 0 runs something else (the
-// encoder's look-back): named barrier 1 over blockDim.x - 32 threads, which all
-// of warps 1.. must reach.  `red` as block_reduce2 (66 entries).  OP as
-// block_reduce.
-__device__ __forceinline__ void sub_sync() { asm volatile("bar.sync 1, %0;" ::"r"(blockDim.x - 32) : "memory"); }
-template <int OPA, int OPB>
-__device__ __forceinline__ void sub_reduce2(u128 &a, u128 &b, u128 *red) {
-  warps_reduce2<OPA, OPB>(a, b, red, (int)(threadIdx.x >> 5) - 1, (int)(blockDim.x >> 5) - 1, [] { sub_sync(); });
-}
-// The same over warps 1.. of a group of G threads (warp 0 of the group runs the
-// look-back): a whole CTA uses named barrier 1, a sub-group g barrier 12 + g.
-template <int G>
-__device__ __forceinline__ void group_sub_sync() {
-  if (GroupOf<G>::sub) asm volatile("bar.sync %0, %1;" ::"r"(12u + threadIdx.x / G), "n"(G - 32) : "memory");
-  else sub_sync();
-}
-template <int OPA, int OPB, int G>
-__device__ __forceinline__ void group_sub_reduce2(u128 &a, u128 &b, u128 *red) {
-  if (GroupOf<G>::sub)
-    warps_reduce2<OPA, OPB>(a, b, red, (int)(group_rank<G>() >> 5) - 1, G / 32 - 1, [] { group_sub_sync<G>(); });
-  else
-    sub_reduce2<OPA, OPB>(a, b, red);
-}
-
 // ---- relaxed global word access for the look-back scan ----------------------
 __device__ __forceinline__ uint64_t ld_relaxed(const uint64_t *p) {
   uint64_t v;

@@ -1,15 +1,7 @@
-// leco_encode.cu -- single-pass column encoder for the LeCo fixed-block codecs.
-//
-// One CTA encodes one block per launch slot:
-//   1. take a block id from a ticket counter (ids are handed out in start order,
-//      so every predecessor of a block is already running or finished),
-//   2. stage the block's values in shared memory (read once from HBM),
-//   3. fit the model, compute residuals and the bit width l,
-//   4. get the block's byte offset from a decoupled look-back prefix sum over
-//      the per-block image sizes (status words in the caller's workspace),
-//   5. write the exact reference block image (header + LSB-first packed body)
-//      straight to its place in the payload with 16-byte stores, byte stores at
-//      the two unaligned ends.
+// leco_encode.cu -- column encode: the dispatch to the row encoder (leco_rows.cuh), the
+// sequential fit kernels of the largest columns, and the legacy u32 codec's kernels (one CTA
+// or one warp per block: stage the values, fit, residuals and width, decoupled look-back for
+// the byte offset, image written straight to its place in the payload).
 //
 // Reference: Leco_int<T>::encodeArray8_int (piecewise_fix_integer_template.h:27-140),
 // FOR_int<T>::encodeArray8_int (FOR_integer_template.h:26-81),
@@ -22,39 +14,33 @@
 
 namespace leco {
 
-// CTAs per SM the encoder's register budget is set for: six (40 registers) for u64 LeCo
-// blocks, whose shared memory allows six, and for the other u32 codecs; five (48) for
-// the other u64 codecs; four (64) for degree-2 blocks.
-template <typename T, int CODEC>
-constexpr int enc_min_ctas() {
-  return CODEC == kPoly2 ? 4 : (sizeof(T) == 4 || CODEC == kLinear) ? 6 : 5;
-}
+int launch_rows_u32(int codec, const EncodeArgs &a, bool ref, cudaStream_t st);
+int launch_rows_u64(int codec, const EncodeArgs &a, bool ref, cudaStream_t st);
 
-template <typename T, int CODEC>
-__global__ void __launch_bounds__(256, enc_min_ctas<T, CODEC>()) encode_kernel(EncodeArgs a) {
+// The legacy u32 codec keeps the block encoder: one CTA per block, block ids from a ticket.
+__global__ void __launch_bounds__(256, 6) encode_legacy_kernel(EncodeArgs a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   __shared__ uint64_t ticket;
   if (threadIdx.x == 0) ticket = atomicAdd(a.ticket, 1u);
   __syncthreads();
   const uint64_t b = ticket;
   if (b >= a.nb) return;
-  encode_block<T, CODEC>(a, b, smem_raw);
+  encode_legacy_block<256>(a, b, smem_raw);
   // block 0 has published its inclusive prefix: its first warp stays on as the prefix
   // publisher for the rest of the column
   if (b == 0 && threadIdx.x < 32 && a.nb > 1) publish_prefixes(a.status, a.nb, a.error);
 }
 
-// Small blocks: one warp per block, eight blocks per CTA, each warp with its
+// Small legacy blocks: one warp per block, eight blocks per CTA, each warp with its
 // own slice of shared memory and its own ticket.
-template <typename T, int CODEC>
-__global__ void __launch_bounds__(256) encode_kernel_warp(EncodeArgs a, uint32_t slice) {
+__global__ void __launch_bounds__(256) encode_legacy_kernel_warp(EncodeArgs a, uint32_t slice) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t t = 0;
   if (lane == 0) t = atomicAdd(a.ticket, 1u);
   const uint64_t b = __shfl_sync(0xffffffffu, t, 0);
   if (b >= a.nb) return;
-  encode_block<T, CODEC, 32>(a, b, smem_raw + (size_t)w * slice);
+  encode_legacy_block<32>(a, b, smem_raw + (size_t)w * slice);
 }
 
 // Sequential reference fits, one warp per 32 blocks: each step the warp loads a
@@ -237,67 +223,62 @@ __global__ void __launch_bounds__(32) seq_fit_ring_kernel(const T *__restrict__ 
 
 // ---- host launchers ---------------------------------------------------------------
 
+// u64 LeCo columns of at least this many blocks take the fits from the kernels below, which
+// read the values once more but run at memory speed (100M values, 24,415 blocks: 190 us), and
+// leave the row encoder without its own (100M: 603 us with the fits inside, 522 us with the
+// fit pass).  A short column's fit kernel is bound by one block's chains of dependent additions
+// (71 us for 4096 values, one block or thousands), which the row encoder does not have.
+constexpr uint64_t kSeqFitBlocks = 16384;
+// The sequential fits of a column's blocks into L.seq_models (CODEC: kLinear, also for the
+// legacy codec, or kPoly2).
 template <typename T, int CODEC>
-static int launch_encode_t(const EncodeLaunch &L, cudaStream_t st) {
-  EncodeArgs a;
-  a.values = L.values; a.n = L.n; a.bs = L.bs; a.nb = L.nb;
-  a.payload = L.payload; a.payload_cap = L.payload_cap; a.offsets = L.offsets; a.dir = L.dir;
-  a.seq_models = nullptr; a.status = L.status; a.ticket = L.ticket; a.error = L.error;
-  // u32 LeCo / degree-2 blocks of 513..4096 values pack their residual rows in an area of
-  // shared memory after the values (six CTAs per SM are set by registers there anyway)
-  a.rows_area = sizeof(T) == 4 && (CODEC == kLinear || CODEC == kPoly2) && L.bs > kWarpBlock && L.bs <= 4096;
+static int launch_seq_fit(const EncodeLaunch &L, cudaStream_t st) {
   PolyX px;
-  for (int i = 0; i < 10; ++i) a.polyX[i] = px.x[i] = L.polyX[i];
-  if (L.seq_models && (CODEC == kLinear || CODEC == kPoly2 || CODEC == kLegacy)) {
-    // four warps per CTA, 32 blocks per warp (the legacy codec fits as LINEAR does)
-    constexpr int FC = CODEC == kLegacy ? kLinear : CODEC;
-    const uint64_t warps = (L.nb + 31) / 32;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (warps <= 4ull * (uint64_t)sms && (reinterpret_cast<uintptr_t>(L.values) & 15) == 0 &&
-        ((uint64_t)L.bs * sizeof(T)) % 16 == 0) {
-      constexpr uint32_t fsm = fit_smem_bytes<T>();
-      if (fsm > 48 * 1024)
-        cudaFuncSetAttribute(seq_fit_ring_kernel<T, FC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm);
-      seq_fit_ring_kernel<T, FC><<<(unsigned)warps, 32, fsm, st>>>(reinterpret_cast<const T *>(L.values), L.n, L.bs,
-                                                                   L.nb, px, L.seq_models);
-    } else {
-      seq_fit_tiled_kernel<T, FC><<<(unsigned)((L.nb + 127) / 128), 128, 0, st>>>(
-          reinterpret_cast<const T *>(L.values), L.n, L.bs, L.nb, px, L.seq_models);
-    }
-    a.seq_models = L.seq_models;
+  for (int i = 0; i < 10; ++i) px.x[i] = L.polyX[i];
+  // four warps per CTA, 32 blocks per warp
+  const uint64_t warps = (L.nb + 31) / 32;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const T *values = reinterpret_cast<const T *>(L.values);
+  if (warps <= 4ull * (uint64_t)sms && (reinterpret_cast<uintptr_t>(L.values) & 15) == 0 && ((uint64_t)L.bs * sizeof(T)) % 16 == 0) {
+    constexpr uint32_t fsm = fit_smem_bytes<T>();
+    if (fsm > 48 * 1024) cudaFuncSetAttribute(seq_fit_ring_kernel<T, CODEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm);
+    seq_fit_ring_kernel<T, CODEC><<<(unsigned)warps, 32, fsm, st>>>(values, L.n, L.bs, L.nb, px, L.seq_models);
+  } else {
+    seq_fit_tiled_kernel<T, CODEC><<<(unsigned)((L.nb + 127) / 128), 128, 0, st>>>(values, L.n, L.bs, L.nb, px, L.seq_models);
   }
-  const uint32_t smem = enc_smem_bytes(L.bs, sizeof(T)) + (a.rows_area ? enc_rows_bytes(L.bs) : 0u);
-  if (L.bs <= kWarpBlock) {
-    const uint32_t slice = (smem + 15) / 16 * 16;
-    encode_kernel_warp<T, CODEC><<<(unsigned)((L.nb + 7) / 8), 256, 8 * slice, st>>>(a, slice);
-    return 0;
-  }
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(encode_kernel<T, CODEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  encode_kernel<T, CODEC><<<(unsigned)L.nb, 256, smem, st>>>(a);
   return 0;
 }
 
 int launch_encode(int codec, int s, const EncodeLaunch &L, cudaStream_t st) {
-  if (s == 4) {
-    switch (codec) {
-      case kLinear: return launch_encode_t<uint32_t, kLinear>(L, st);
-      case kFor: return launch_encode_t<uint32_t, kFor>(L, st);
-      case kDelta: return launch_encode_t<uint32_t, kDelta>(L, st);
-      case kPoly2: return launch_encode_t<uint32_t, kPoly2>(L, st);
-      case kLegacy: return launch_encode_t<uint32_t, kLegacy>(L, st);
+  EncodeArgs a;
+  a.values = L.values; a.n = L.n; a.bs = L.bs; a.nb = L.nb;
+  a.payload = L.payload; a.payload_cap = L.payload_cap; a.offsets = L.offsets; a.dir = L.dir;
+  a.seq_models = nullptr; a.status = L.status; a.ticket = L.ticket; a.error = L.error;
+  for (int i = 0; i < 10; ++i) a.polyX[i] = L.polyX[i];
+  if (codec != kLegacy) {
+    const bool ref = L.seq_models != nullptr;
+    if (ref && codec == kLinear && s == 8 && L.nb >= kSeqFitBlocks) {
+      launch_seq_fit<uint64_t, kLinear>(L, st);
+      a.seq_models = L.seq_models;
     }
-  } else {
-    switch (codec) {
-      case kLinear: return launch_encode_t<uint64_t, kLinear>(L, st);
-      case kFor: return launch_encode_t<uint64_t, kFor>(L, st);
-      case kDelta: return launch_encode_t<uint64_t, kDelta>(L, st);
-      case kPoly2: return launch_encode_t<uint64_t, kPoly2>(L, st);
-    }
+    return s == 4 ? launch_rows_u32(codec, a, ref, st) : launch_rows_u64(codec, a, ref, st);
   }
-  return -1;
+  if (s != 4) return -1;
+  if (L.seq_models) {  // the legacy codec fits as LINEAR does
+    launch_seq_fit<uint32_t, kLinear>(L, st);
+    a.seq_models = L.seq_models;
+  }
+  const uint32_t smem = enc_smem_bytes(L.bs, 4);
+  if (L.bs <= kWarpBlock) {
+    const uint32_t slice = (smem + 15) / 16 * 16;
+    encode_legacy_kernel_warp<<<(unsigned)((L.nb + 7) / 8), 256, 8 * slice, st>>>(a, slice);
+    return 0;
+  }
+  if (smem > 48 * 1024) cudaFuncSetAttribute(encode_legacy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  encode_legacy_kernel<<<(unsigned)L.nb, 256, smem, st>>>(a);
+  return 0;
 }
 
 // Bounded-wait check: block 1 of a two-block look-back whose block 0 never

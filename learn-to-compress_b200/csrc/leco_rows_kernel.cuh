@@ -1,0 +1,53 @@
+// leco_rows_kernel.cuh -- the single-column kernel of the row encoder, instantiated per value
+// type in leco_rows_u32.cu and leco_rows_u64.cu.
+#pragma once
+#include "leco_rows.cuh"
+
+namespace leco {
+
+// CTAs per SM the registers are budgeted for: what the rows' shared memory allows (six of four
+// warps with u64 LeCo rows, eight with u32 rows), capped at 1024 threads per SM.
+template <typename T, int CODEC, int NT>
+constexpr int rows_min_ctas() {
+  if (sizeof(T) == 8) return CODEC == kPoly2 ? (NT == 128 ? 5 : NT == 256 ? 2 : 1) : (NT == 128 ? 6 : NT == 256 ? 3 : 1);
+  if (CODEC == kPoly2) return NT == 128 ? 6 : NT == 256 ? 3 : 1;
+  return CODEC == kLinear ? (NT == 128 ? 8 : NT == 256 ? 4 : 2) : (NT == 128 ? 10 : NT == 256 ? 5 : 2);
+}
+
+// One CTA of NT threads per item of NT / R blocks (RT: R when it is 64 or more, else 0).  A
+// column of one item needs no other; else CTA 0 is the publisher and CTA i + 1 takes item i:
+// CTAs start in the order of their index, so the publisher runs before any item and every
+// item it waits for has started.
+template <typename T, int CODEC, int NT, uint32_t RT>
+__global__ void __launch_bounds__(NT, rows_min_ctas<T, CODEC, NT>()) encode_rows_kernel(EncodeArgs a, uint32_t R, uint32_t items,
+                                                                                         bool ref) {
+  extern __shared__ __align__(256) uint8_t smem_raw[];
+  if (items > 1 && blockIdx.x == 0) publish_items<NT>(a.status, items, a.error, smem_raw);
+  else encode_rows_item<T, CODEC, RT, true>(a, items > 1 ? blockIdx.x - 1 : 0, R, ref, items == 1, smem_raw);
+}
+
+template <typename T, int CODEC, int NT, uint32_t RT>
+int launch_rows_nt(const EncodeArgs &a, uint32_t R, bool ref, cudaStream_t st) {
+  const uint64_t nb_item = NT / R, items = (a.nb + nb_item - 1) / nb_item;
+  const uint32_t smem = rows_layout(NT, R, sizeof(T), rows_sums(CODEC)).total;
+  if (smem > 48 * 1024) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(encode_rows_kernel<T, CODEC, NT, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return -(int)e;
+  }
+  encode_rows_kernel<T, CODEC, NT, RT><<<(unsigned)(items > 1 ? items + 1 : 1), NT, smem, st>>>(a, R, (uint32_t)items, ref);
+  return 0;
+}
+template <typename T, int CODEC>
+int launch_rows_t(const EncodeArgs &a, bool ref, cudaStream_t st) {
+  const uint32_t R = rows_threads(a.bs);
+  switch (R) {
+    case 64: return launch_rows_nt<T, CODEC, 128, 64>(a, R, ref, st);
+    case 128: return launch_rows_nt<T, CODEC, 128, 128>(a, R, ref, st);
+    case 256: return launch_rows_nt<T, CODEC, 256, 256>(a, R, ref, st);
+    case 512: return launch_rows_nt<T, CODEC, 512, 512>(a, R, ref, st);
+    default: return launch_rows_nt<T, CODEC, 128, 0>(a, R, ref, st);
+  }
+}
+
+}  // namespace leco
