@@ -13,13 +13,18 @@
 //   2. pairwise merges while the fitted byte size of a pair is below the sum of the
 //      two, pass after pass, until a pass saves less than 0.01 % of the coarse
 //      block's raw size.
-// Both phases are sequential inside a coarse block (every step depends on the
-// previous merge), so the parallelism is across coarse blocks: one thread per
-// coarse block, persistent threads taking blocks by ticket, each with a private
-// scratch slot in global memory (the segment list of phase 1, then the segment
-// starts and sizes of phase 2, merged in place).  Every FP64 step is the
-// reference's, one rounding each (--fmad=false), so the segment starts are the
-// host partitioner's bit for bit.
+// Every merge changes what the next step sees, but most steps merge nothing: of a
+// 2000-value coarse block's ~24,000 list steps ~2,000 are attempts and ~120 merges (the
+// variable-length benchmark's column), and a pass of phase 2 decides on pair sizes that
+// depend only on the segmentation before the pass.  Coarse blocks of up to kPartWarpMax
+// values therefore take one warp each (partition_warp_kernel): the warp tries 32 segments
+// at a time and stops at the first that merges, and computes a pass's pair sizes one per
+// lane, or one by the whole warp when the pair is long.  Larger ones take one thread per
+// coarse block (partition_kernel), persistent threads taking blocks by ticket, each with
+// a private scratch slot in global memory (the segment list of phase 1, then the segment
+// starts and sizes of phase 2, merged in place).  Every FP64 step is the reference's, one
+// rounding each (--fmad=false), so the segment starts are the host partitioner's bit for
+// bit.
 //
 // Output: each coarse block's segment starts go to stage[B0 ...] (at most one per
 // value) with their count; a scan of the counts and a gather compact them into the
@@ -29,6 +34,7 @@
 
 #include "leco_device.cuh"
 #include "leco_internal.h"
+#include "leco_seqsum.cuh"
 
 namespace leco {
 
@@ -287,6 +293,357 @@ __global__ void __launch_bounds__(kPartThreads) partition_kernel(PartitionArgs a
   }
 }
 
+// ---- one warp per coarse block --------------------------------------------------------
+// Phase 1 needs no list.  Segments tile the positions 0 .. len-2 (position p carries the
+// first difference D[p] = y[p+1] - y[p]), so a bitmap of the positions where a segment ends
+// is the list; a segment ending at e has the bit class of D[e], D[e+1] and the difference
+// D[e] to its successor, whatever it has absorbed, and starts after the bit before e.  Only
+// the extremes of the differences inside a merged segment are kept, in global memory at
+// its end (single points have none).  Phase 2 keeps 16-bit starts, sizes and pair sizes;
+// a pair's size is computed again only when one of the two segments has changed.
+// Shared memory: 14 bytes a value, eight warps per SM for blocks of 2000 values.  10M
+// values, 5000 blocks of 2000: 42.8 ms with a thread per block; the figure with a warp per
+// block is at the launch.
+constexpr uint32_t kPartWarpMax = 8000;  // sizes fit 16 bits, shared memory fits an SM twice
+constexpr uint32_t kPartLaneMax = 48;    // pairs of up to this many values: one lane each
+constexpr uint16_t kNoSize = 0xffffu;
+
+struct PartShared {
+  uint64_t *y;
+  uint16_t *idx, *sz, *pc;
+  uint8_t *cls;    // phase 1 (over sz)
+  uint32_t *bits;  // phase 1: segment ends
+};
+__host__ __device__ inline uint32_t part_smem_bytes(uint32_t bs) {
+  const uint32_t list = ((bs + 2) * 2 + 7) / 8 * 8;
+  return bs * 8 + 3 * list + (bs / 32 + 2) * 4;
+}
+__device__ __forceinline__ PartShared part_shared(uint8_t *smem, uint32_t bs) {
+  const uint32_t list = ((bs + 2) * 2 + 7) / 8 * 8;
+  PartShared P;
+  P.y = reinterpret_cast<uint64_t *>(smem);
+  uint8_t *p = smem + (size_t)bs * 8;
+  P.idx = reinterpret_cast<uint16_t *>(p);
+  P.sz = reinterpret_cast<uint16_t *>(p + list);
+  P.pc = reinterpret_cast<uint16_t *>(p + 2 * list);
+  P.cls = p + list;
+  P.bits = reinterpret_cast<uint32_t *>(p + 3 * list);
+  return P;
+}
+
+// cal_bits with the ceiling of half the difference as an integer where that is exact.
+__device__ __forceinline__ int cal_bits_fast(int64_t mn, int64_t mx) {
+  const int64_t diff = (int64_t)((uint64_t)mx - (uint64_t)mn);
+  const uint64_t ad = diff < 0 ? 0 - (uint64_t)diff : (uint64_t)diff;
+  if (ad >= (1ull << 53)) return cal_bits_d(mn, mx);
+  return ad ? (int)bits64_d((ad + 1) >> 1) + 1 : 0;
+}
+// The segment end before position e (-1: none) and the one after it (one exists).
+__device__ __forceinline__ int part_prev(const uint32_t *bits, int e) {
+  int w = e >> 5;
+  uint32_t v = bits[w] & ((1u << (e & 31)) - 1u);
+  while (!v) {
+    if (--w < 0) return -1;
+    v = bits[w];
+  }
+  return 32 * w + 31 - __clz((int)v);
+}
+__device__ __forceinline__ int part_next(const uint32_t *bits, int e) {
+  int w = (e + 1) >> 5;
+  uint32_t v = bits[w] & (0xffffffffu << ((e + 1) & 31));
+  while (!v) v = bits[++w];
+  return 32 * w + __ffs((int)v) - 1;
+}
+// Size of a segment of `length` >= 3 values from its largest residual.
+__device__ __forceinline__ uint32_t part_size(uint64_t maxr, uint32_t length) {
+  const uint32_t bits = maxr ? bits64_d(maxr) + 1 : 0;
+  if (bits >= 64) return 5 + 8 * length;
+  return 17 + (bits * length + 7) / 8;
+}
+__device__ __forceinline__ void part_model(double sumy, double sumxy, uint32_t length, double &t0, double &slope) {
+  const uint64_t m = length;
+  const double dm = __uint2double_rn(length);
+  // sum i and sum i*i are exact integers at every step of the reference's loop
+  const double sumx = __ull2double_rn(m * (m - 1) / 2), sumxx = __ull2double_rn((m - 1) * m * (2 * m - 1) / 6);
+  const double ccc = __dsub_rn(__dmul_rn(sumxy, dm), __dmul_rn(sumx, sumy));
+  const double xxx = __dsub_rn(__dmul_rn(sumxx, dm), __dmul_rn(sumx, sumx));
+  const double t1 = __ddiv_rn(ccc, xxx);
+  t0 = __ddiv_rn(__dsub_rn(sumy, __dmul_rn(t1, sumx)), dm);
+  slope = (double)__double2float_rn(t1);
+}
+// The largest residual of values first, first + step, ... of a segment (128-bit predictions,
+// 64-bit ones where the ends say that every prediction lies in [0, 2^63)).
+__device__ __forceinline__ uint64_t part_residual(const uint64_t *y, uint32_t length, uint32_t first, uint32_t step, double t0,
+                                                  double slope) {
+  const double p0 = __dadd_rn(t0, __dmul_rn(slope, 0.0)), p1 = __dadd_rn(t0, __dmul_rn(slope, __uint2double_rn(length - 1)));
+  const bool narrow = p0 >= 0.0 && p1 >= 0.0 && p0 < 9223372036854775808.0 && p1 < 9223372036854775808.0;
+  uint64_t maxr = 0;
+  if (narrow) {
+#pragma unroll 2
+    for (uint32_t j = first; j < length; j += step) {
+      const uint64_t pred = __double2ull_rz(__dadd_rn(t0, __dmul_rn(slope, u32_to_double_fp64(j)))), v = y[j];
+      const uint64_t r = v > pred ? v - pred : pred - v;
+      maxr = r > maxr ? r : maxr;
+    }
+  } else {
+    for (uint32_t j = first; j < length; j += step) {
+      const i128 pred = f2i128(__dadd_rn(t0, __dmul_rn(slope, u32_to_double_fp64(j)))), v = (i128)y[j];
+      const uint64_t r = (uint64_t)(v > pred ? v - pred : pred - v);
+      maxr = r > maxr ? r : maxr;
+    }
+  }
+  return maxr;
+}
+// newsegment_size of y[0 .. length), one lane.
+__device__ __forceinline__ uint32_t lane_size(const uint64_t *y, uint32_t length) {
+  if (length == 1) return 9;
+  if (length == 2) return 13;
+  double sumy = 0, sumxy = 0, k = 0;
+#pragma unroll 4
+  for (uint32_t i = 0; i < length; i++) {
+    const double v = u64_to_double_fp64(y[i]);
+    sumy = __dadd_rn(sumy, v);
+    sumxy = __dadd_rn(sumxy, __dmul_rn(k, v));
+    k = __dadd_rn(k, 1.0);
+  }
+  double t0, slope;
+  part_model(sumy, sumxy, length, t0, slope);
+  return part_size(part_residual(y, length, 0, 1, t0, slope), length);
+}
+// The same by the whole warp.
+__device__ __noinline__ uint32_t warp_size(const uint64_t *y, uint32_t length) {
+  double sumy, sumxy, t0, slope;
+  warp_seq_sums(y, length, sumy, sumxy);
+  part_model(sumy, sumxy, length, t0, slope);
+  return part_size(warp_max_u64(part_residual(y, length, threadIdx.x & 31, 32, t0, slope)), length);
+}
+
+// Phase 1 of a coarse block of len >= 2 values; mm: the merged segments' (min, max)
+// differences, at their ends.
+__device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t len, int overhead, longlong2 *mm) {
+  const int lane = threadIdx.x & 31, last = (int)len - 2;  // the last segment's end
+  const uint64_t *y = P.y;
+  int lo = 10000, hi = -1;
+  for (int p = lane; p < last; p += 32) {
+    const int64_t d0 = (int64_t)(y[p + 1] - y[p]), d1 = (int64_t)(y[p + 2] - y[p + 1]);
+    const int c = cal_bits_fast(d0, d1);
+    P.cls[p] = (uint8_t)c;
+    lo = min(lo, c);
+    hi = max(hi, c);
+  }
+  if (lane == 0) P.cls[last] = (uint8_t)kNoClass;
+  const int words = (last >> 5) + 1;
+  for (int w = lane; w < words; w += 32) P.bits[w] = 32 * w + 31 <= last ? 0xffffffffu : (2u << (last & 31)) - 1u;
+  for (int m = 16; m; m >>= 1) {
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, m));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, m));
+  }
+  __syncwarp();
+  auto diff = [&](int p) { return (int64_t)(y[p + 1] - y[p]); };
+  auto extremes = [&](int s, int e) { return s == e ? make_longlong2(0, 0) : mm[e]; };  // of segment [s, e]
+  for (int aim = lo; aim <= hi; ++aim) {
+    int from = 0;  // segments that end before it have had their turn
+    for (int w = 0; w < words;) {
+      const int e = 32 * w + lane;
+      const bool match = e >= from && e < last && ((P.bits[w] >> lane) & 1u) && P.cls[e] == (uint8_t)aim;
+      if (!__any_sync(0xffffffffu, match)) {
+        ++w;
+        continue;
+      }
+      // segment c = [s, e] with its right neighbour [e + 1, en]
+      int s = 0, en = 0;
+      int64_t nmin = 0, nmax = 0;
+      bool merge = false;
+      if (match) {
+        s = part_prev(P.bits, e) + 1;
+        en = part_next(P.bits, e);
+        const longlong2 c = extremes(s, e), n = extremes(e + 1, en);
+        const int64_t d = diff(e);
+        nmax = max(max((int64_t)c.y, (int64_t)n.y), d);
+        nmin = min(min((int64_t)c.x, (int64_t)n.x), d);
+        const int origin = (e + 1 - s) * cal_bits_fast(c.x, c.y) + (en - e) * cal_bits_fast(n.x, n.y);
+        merge = cal_bits_fast(nmin, nmax) * (en - s + 1) - origin < overhead;
+      }
+      const uint32_t hit = __ballot_sync(0xffffffffu, merge);
+      if (!hit) {
+        ++w;
+        continue;
+      }
+      const int f = __ffs((int)hit) - 1;  // the first segment that merges; those before it stay as they are
+      int cs = __shfl_sync(0xffffffffu, s, f), ce = __shfl_sync(0xffffffffu, en, f);
+      int64_t cmin = __shfl_sync(0xffffffffu, (long long)nmin, f), cmax = __shfl_sync(0xffffffffu, (long long)nmax, f);
+      if (lane == 0) P.bits[w] &= ~(1u << f);
+      __syncwarp();
+      // grow left (never into the first segment of the block)
+      while (cs > 0) {
+        const int pe = cs - 1, ps = part_prev(P.bits, pe) + 1;
+        if (ps == 0) break;
+        const longlong2 p = extremes(ps, pe);
+        const int64_t d = diff(pe);
+        const int64_t lmax = max(max((int64_t)p.y, cmax), d), lmin = min(min((int64_t)p.x, cmin), d);
+        const int oc = (cs - ps) * cal_bits_fast(p.x, p.y) + (ce - cs + 1) * cal_bits_fast(cmin, cmax);
+        if (!(cal_bits_fast(lmin, lmax) * (ce - ps + 1) - oc < overhead)) break;
+        __syncwarp();  // every lane has read the bits
+        if (lane == 0) P.bits[pe >> 5] &= ~(1u << (pe & 31));
+        __syncwarp();
+        cs = ps;
+        cmin = lmin;
+        cmax = lmax;
+      }
+      // grow right (never into the last segment of the block)
+      while (ce < last) {
+        const int ne = part_next(P.bits, ce);
+        if (ne == last) break;
+        const longlong2 n = extremes(ce + 1, ne);
+        const int64_t d = diff(ce);
+        const int64_t rmax = max(max((int64_t)n.y, cmax), d), rmin = min(min((int64_t)n.x, cmin), d);
+        const int oc = (ne - ce) * cal_bits_fast(n.x, n.y) + (ce + 1 - cs) * cal_bits_fast(cmin, cmax);
+        if (!(cal_bits_fast(rmin, rmax) * (ne - cs + 1) - oc < overhead)) break;
+        __syncwarp();
+        if (lane == 0) P.bits[ce >> 5] &= ~(1u << (ce & 31));
+        __syncwarp();
+        ce = ne;
+        cmin = rmin;
+        cmax = rmax;
+      }
+      __syncwarp();
+      if (lane == 0) mm[ce] = make_longlong2(cmin, cmax);
+      __syncwarp();
+      from = ce + 1;
+      w = from >> 5;
+    }
+  }
+}
+
+// Fills out[k] for k < count where it holds kNoSize: the size of y[at(k) .. end(k)).
+template <typename At, typename End>
+__device__ __forceinline__ void part_sizes(const uint64_t *y, uint16_t *out, uint32_t count, At at, End end) {
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t k0 = 0; k0 < count; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    const bool need = k < count && out[k] == kNoSize;
+    const uint32_t s = need ? at(k) : 0, length = need ? end(k) - s : 0;
+    if (need && length <= kPartLaneMax) out[k] = (uint16_t)lane_size(y + s, length);
+    uint32_t rest = __ballot_sync(0xffffffffu, need && length > kPartLaneMax);
+    while (rest) {
+      const int f = __ffs((int)rest) - 1;
+      rest &= rest - 1;
+      const uint32_t fs = __shfl_sync(0xffffffffu, s, f), fl = __shfl_sync(0xffffffffu, length, f);
+      const uint32_t z = warp_size(y + fs, fl);
+      if ((int)lane == f) out[k] = (uint16_t)z;
+    }
+  }
+  __syncwarp();
+}
+
+// Phase 2: the pairwise merge passes; returns the number of segments, their starts in P.idx.
+__device__ __forceinline__ uint32_t part_merge_pairs(const PartShared &P, uint32_t len, uint32_t bs) {
+  const uint32_t lane = threadIdx.x & 31, last = len - 2;
+  const uint32_t below = (1u << lane) - 1u;
+  // starts: 0 and each end but the last, plus one
+  uint32_t m = 1;
+  if (lane == 0) P.idx[0] = 0;
+  for (uint32_t w = 0; w <= last >> 5; ++w) {
+    uint32_t v = P.bits[w];
+    if (w == last >> 5) v &= ~(1u << (last & 31));
+    if ((v >> lane) & 1u) P.idx[m + __popc(v & below)] = (uint16_t)(32 * w + lane + 1);
+    m += __popc(v);
+  }
+  __syncwarp();
+  if (lane == 0) P.idx[m] = P.idx[m + 1] = (uint16_t)len;  // ends of the last segment and of the last pair
+  for (uint32_t k = lane; k < m; k += 32) {
+    P.sz[k] = kNoSize;
+    P.pc[k] = kNoSize;
+  }
+  __syncwarp();
+  auto start = [&](uint32_t k) -> uint32_t { return P.idx[k]; };
+  part_sizes(P.y, P.sz, m, start, [&](uint32_t k) -> uint32_t { return P.idx[k + 1]; });
+  uint64_t total = 0;
+  for (uint32_t k = lane; k < m; k += 32) total += P.sz[k];
+  total = warp_sum_u64(total);
+  for (;;) {
+    part_sizes(P.y, P.pc, m - 1, start, [&](uint32_t k) -> uint32_t { return P.idx[k + 2]; });
+    // From the left: a pair whose size is smaller than its parts' merges and is passed over,
+    // so in a run of such pairs every other one merges, from the run's first on.
+    uint32_t w = 0;          // segments of the new list
+    uint32_t taken = 0;      // 1: the first segment of this group went into the pair before it
+    uint64_t tnew = 0;
+    // (entries of the list are written no further on than they were read: the group's own
+    // are in registers, and w <= k0; the next group's first pair flag is taken ahead)
+    for (uint32_t k0 = 0; k0 < m; k0 += 32) {
+      const uint32_t k = k0 + lane;
+      const uint32_t z = k < m ? P.sz[k] : 0, q = k + 1 < m ? P.pc[k] : kNoSize;
+      const uint32_t z1 = k + 1 < m ? P.sz[k + 1] : 0, i0 = k < m ? P.idx[k] : 0;
+      const bool want = k + 1 < m && z + z1 > q;
+      uint32_t f = __ballot_sync(0xffffffffu, want) & ~taken;
+      const uint32_t even = 0x55555555u, run0 = f & ~(f << 1);
+      const uint32_t from_even = f & ~(f + (run0 & even));  // the runs that begin at an even place
+      const uint32_t merge = (from_even & even) | ((f & ~from_even) & ~even);
+      const uint32_t gone = (merge << 1) | taken, in = m - k0 >= 32 ? 0xffffffffu : (1u << (m - k0)) - 1u;
+      const uint32_t keep = ~gone & in;
+      // the pair (k, k + 1) stays a pair when neither merges (k + 1's flag may be the next group's)
+      const uint32_t k1 = k0 + 32;
+      uint32_t next_merges = 0;
+      if (!(merge >> 31) && k1 < m) {  // segment k1 is free: does it merge?
+        const uint32_t a = P.sz[k1], b = k1 + 1 < m ? P.sz[k1 + 1] : 0, c = k1 + 1 < m ? P.pc[k1] : kNoSize;
+        next_merges = k1 + 1 < m && a + b > c;
+      }
+      const uint32_t after = (merge >> 1) | (next_merges << 31);  // does segment k + 1 merge
+      __syncwarp();
+      if ((keep >> lane) & 1u) {
+        const uint32_t o = w + __popc(keep & below);
+        const bool mg = (merge >> lane) & 1u;
+        const uint32_t nz = mg ? q : z;
+        P.idx[o] = (uint16_t)i0;
+        P.sz[o] = (uint16_t)nz;
+        P.pc[o] = mg || ((after >> lane) & 1u) ? kNoSize : (uint16_t)q;
+        tnew += nz;
+      }
+      w += __popc(keep);
+      taken = merge >> 31;
+      __syncwarp();
+    }
+    m = w;
+    if (lane == 0) P.idx[m] = P.idx[m + 1] = (uint16_t)len;
+    __syncwarp();
+    tnew = warp_sum_u64(tnew);
+    const uint64_t decline = total - tnew;  // unsigned, as in the reference
+    total = tnew;
+    const double pct = __ddiv_rn(__dmul_rn(__ull2double_rn(decline), 100.0), __dmul_rn((double)sizeof(uint64_t), (double)bs));
+    if (!(decline > 0) || pct < 0.01) break;
+  }
+  return m;
+}
+
+__global__ void __launch_bounds__(32) partition_warp_kernel(PartitionArgs a) {
+  extern __shared__ __align__(16) uint8_t part_smem[];
+  const uint32_t lane = threadIdx.x;
+  const PartShared P = part_shared(part_smem, a.bs);
+  longlong2 *mm = reinterpret_cast<longlong2 *>(a.segs) + (size_t)blockIdx.x * a.bs;
+  for (;;) {
+    uint32_t t = 0;
+    if (lane == 0) t = atomicAdd(a.ticket, 1u);
+    const uint64_t b = __shfl_sync(0xffffffffu, t, 0);
+    if (b >= a.nblocks) return;
+    const uint64_t B0 = b * a.bs;
+    const uint32_t len = (uint32_t)(b == a.nblocks - 1 ? a.n - B0 : a.bs);
+    if (len < 2) {  // the reference needs two points per coarse block (it reads array[B0 + 1])
+      if (lane == 0) {
+        a.stage[B0] = (uint32_t)B0;
+        a.count[b] = 1;
+      }
+      continue;
+    }
+    for (uint32_t i = lane; i < len; i += 32) P.y[i] = __ldg(a.array + B0 + i);
+    __syncwarp();
+    part_merge_classes(P, len, a.overhead, mm);
+    const uint32_t m = part_merge_pairs(P, len, a.bs);
+    for (uint32_t k = lane; k < m; k += 32) a.stage[B0 + k] = (uint32_t)B0 + P.idx[k];
+    if (lane == 0) a.count[b] = m;
+    __syncwarp();
+  }
+}
+
 // Exclusive scan of the per-block counts (one CTA, chunks of 1024), then each
 // block's starts are copied to their place in the caller's array.
 __global__ void __launch_bounds__(1024) count_scan_kernel(const uint32_t *count, uint64_t nb, uint64_t *base, uint64_t *total) {
@@ -403,7 +760,23 @@ int leco_varlen_partition_device(const uint64_t *d_values, uint64_t n, uint32_t 
   A.ticket = reinterpret_cast<uint32_t *>(w);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(A.ticket, 0, 4, st) != cudaSuccess) return record_error(LECO_ERR_CUDA, "leco_varlen_partition_device: memset");
-  partition_kernel<<<(unsigned)(slots / kPartThreads), kPartThreads, 0, st>>>(A);
+  if (bs <= kPartWarpMax) {
+    const uint32_t smem = part_smem_bytes(bs);
+    cudaError_t se = cudaSuccess;
+    if (smem > 48 * 1024)
+      se = cudaFuncSetAttribute(partition_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    int dev = 0, sms = 148, per_sm = 1;
+    if (se == cudaSuccess) se = cudaGetDevice(&dev);
+    if (se == cudaSuccess) se = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (se == cudaSuccess) se = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, partition_warp_kernel, 32, smem);
+    if (se != cudaSuccess)
+      return record_error(LECO_ERR_CUDA, std::string("leco_varlen_partition_device: ") + cudaGetErrorString(se));
+    // a warp's scratch (16 bytes a value) lies in its slot's segment list (48 bytes a value): no more warps than slots
+    const uint64_t grid = std::min<uint64_t>(std::min<uint64_t>(nb, slots), (uint64_t)sms * (uint64_t)std::max(per_sm, 1));
+    partition_warp_kernel<<<(unsigned)grid, 32, smem, st>>>(A);
+  } else {
+    partition_kernel<<<(unsigned)(slots / kPartThreads), kPartThreads, 0, st>>>(A);
+  }
   count_scan_kernel<<<1, 1024, 0, st>>>(A.count, nb, base, d_nseg);
   starts_gather_kernel<<<(unsigned)std::min<uint64_t>(nb, 148 * 8), 256, 0, st>>>(A.stage, A.count, base, nb, bs, d_starts,
                                                                                    starts_cap, err);
