@@ -16,10 +16,10 @@
 // Every merge changes what the next step sees, but most steps merge nothing: of a
 // 2000-value coarse block's ~24,000 list steps ~2,000 are attempts and ~120 merges (the
 // variable-length benchmark's column), and a pass of phase 2 decides on pair sizes that
-// depend only on the segmentation before the pass.  Coarse blocks of up to kPartWarpMax
-// values therefore take one warp each (partition_warp_kernel): the warp tries 32 segments
-// at a time and stops at the first that merges, and computes a pass's pair sizes one per
-// lane, or one by the whole warp when the pair is long.  Larger ones take one thread per
+// depend only on the segmentation before the pass.  Coarse blocks of up to kPartCtaMax
+// values therefore take one CTA each (partition_cta_kernel): a warp tries 32 segments at
+// a time and stops at the first that merges, and the CTA's warps compute a pass's pair
+// sizes one per lane, or one by a whole warp when the pair is long.  Larger ones take one thread per
 // coarse block (partition_kernel), persistent threads taking blocks by ticket, each with
 // a private scratch slot in global memory (the segment list of phase 1, then the segment
 // starts and sizes of phase 2, merged in place).  Every FP64 step is the reference's, one
@@ -293,41 +293,51 @@ __global__ void __launch_bounds__(kPartThreads) partition_kernel(PartitionArgs a
   }
 }
 
-// ---- one warp per coarse block --------------------------------------------------------
+// ---- one CTA per coarse block ---------------------------------------------------------
 // Phase 1 needs no list.  Segments tile the positions 0 .. len-2 (position p carries the
 // first difference D[p] = y[p+1] - y[p]), so a bitmap of the positions where a segment ends
 // is the list; a segment ending at e has the bit class of D[e], D[e+1] and the difference
 // D[e] to its successor, whatever it has absorbed, and starts after the bit before e.  Only
 // the extremes of the differences inside a merged segment are kept, in global memory at
-// its end (single points have none).  Phase 2 keeps 16-bit starts, sizes and pair sizes;
-// a pair's size is computed again only when one of the two segments has changed.
-// Shared memory: 14 bytes a value, eight warps per SM for blocks of 2000 values.  10M
-// values, 5000 blocks of 2000: 42.8 ms with a thread per block; the figure with a warp per
-// block is at the launch.
-constexpr uint32_t kPartWarpMax = 8000;  // sizes fit 16 bits, shared memory fits an SM twice
+// its end (single points have none).  The positions are sorted by bit class once, so that a
+// class's turn visits its own positions only, 32 at a time; a position that has been
+// absorbed is skipped.  Phase 2 keeps 16-bit starts, sizes and pair sizes; a pair's size is
+// computed again only when one of the two segments has changed.
+// Bound by latency: phase 1 is one warp's, phase 2 mostly sums of the fits.  Shared memory:
+// 14 bytes a value, eight CTAs per SM for blocks of 2000 values.  10M values, 5000 blocks of
+// 2000, partition and encode: 43.7 ms with a thread per block, 4.47 ms with one warp per
+// block that scanned every class over all positions, 2.59 ms now.
+constexpr uint32_t kPartCtaMax = 8000;   // sizes fit 16 bits, shared memory fits an SM twice
 constexpr uint32_t kPartLaneMax = 48;    // pairs of up to this many values: one lane each
+constexpr uint32_t kPartWarps = 4;
 constexpr uint16_t kNoSize = 0xffffu;
 
 struct PartShared {
   uint64_t *y;
   uint16_t *idx, *sz, *pc;
-  uint8_t *cls;    // phase 1 (over sz)
-  uint32_t *bits;  // phase 1: segment ends
+  uint16_t *order;  // phase 1 (over idx): positions by class
+  uint8_t *cls;     // phase 1 (over sz)
+  uint32_t *bits;   // phase 1: segment ends
+  uint32_t *hist;   // phase 1: [72] where a class's positions end in order; phase 2: [0] long pairs, [1] segments, [2] done
+  uint16_t *jobs;   // phase 2 (over bits): pairs that take a warp
 };
+__host__ __device__ inline uint32_t part_list_bytes(uint32_t bs) { return ((bs + 2) * 2 + 7) / 8 * 8; }
+__host__ __device__ inline uint32_t part_jobs_bytes(uint32_t bs) { return (bs / 32 + 2) * 4 + (bs / kPartLaneMax + 4) * 2 * 2; }
 __host__ __device__ inline uint32_t part_smem_bytes(uint32_t bs) {
-  const uint32_t list = ((bs + 2) * 2 + 7) / 8 * 8;
-  return bs * 8 + 3 * list + (bs / 32 + 2) * 4;
+  return bs * 8 + 3 * part_list_bytes(bs) + 72 * 4 + part_jobs_bytes(bs);
 }
 __device__ __forceinline__ PartShared part_shared(uint8_t *smem, uint32_t bs) {
-  const uint32_t list = ((bs + 2) * 2 + 7) / 8 * 8;
+  const uint32_t list = part_list_bytes(bs);
   PartShared P;
   P.y = reinterpret_cast<uint64_t *>(smem);
   uint8_t *p = smem + (size_t)bs * 8;
-  P.idx = reinterpret_cast<uint16_t *>(p);
+  P.idx = P.order = reinterpret_cast<uint16_t *>(p);
   P.sz = reinterpret_cast<uint16_t *>(p + list);
   P.pc = reinterpret_cast<uint16_t *>(p + 2 * list);
   P.cls = p + list;
-  P.bits = reinterpret_cast<uint32_t *>(p + 3 * list);
+  P.hist = reinterpret_cast<uint32_t *>(p + 3 * list);
+  P.bits = P.hist + 72;
+  P.jobs = reinterpret_cast<uint16_t *>(P.bits);
   return P;
 }
 
@@ -418,43 +428,62 @@ __device__ __noinline__ uint32_t warp_size(const uint64_t *y, uint32_t length) {
   return part_size(warp_max_u64(part_residual(y, length, threadIdx.x & 31, 32, t0, slope)), length);
 }
 
-// Phase 1 of a coarse block of len >= 2 values; mm: the merged segments' (min, max)
-// differences, at their ends.
-__device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t len, int overhead, longlong2 *mm) {
-  const int lane = threadIdx.x & 31, last = (int)len - 2;  // the last segment's end
+// Classes of a coarse block of len >= 2 values, every position a segment; by the whole CTA.
+__device__ __forceinline__ void part_classes(const PartShared &P, uint32_t len) {
+  const int last = (int)len - 2;  // the last segment's end
   const uint64_t *y = P.y;
-  int lo = 10000, hi = -1;
-  for (int p = lane; p < last; p += 32) {
+  for (int p = threadIdx.x; p < last; p += blockDim.x) {
     const int64_t d0 = (int64_t)(y[p + 1] - y[p]), d1 = (int64_t)(y[p + 2] - y[p + 1]);
     const int c = cal_bits_fast(d0, d1);
     P.cls[p] = (uint8_t)c;
-    lo = min(lo, c);
-    hi = max(hi, c);
+    atomicAdd(&P.hist[c], 1u);
   }
-  if (lane == 0) P.cls[last] = (uint8_t)kNoClass;
   const int words = (last >> 5) + 1;
-  for (int w = lane; w < words; w += 32) P.bits[w] = 32 * w + 31 <= last ? 0xffffffffu : (2u << (last & 31)) - 1u;
-  for (int m = 16; m; m >>= 1) {
-    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, m));
-    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, m));
+  for (int w = threadIdx.x; w < words; w += blockDim.x) P.bits[w] = 32 * w + 31 <= last ? 0xffffffffu : (2u << (last & 31)) - 1u;
+}
+
+// Phase 1, by one warp; mm: the merged segments' (min, max) differences, at their ends.
+__device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t len, int overhead, longlong2 *mm) {
+  const int lane = threadIdx.x & 31, last = (int)len - 2;
+  const uint64_t *y = P.y;
+  // positions by class, in order within a class
+  uint32_t carry = 0;
+  for (int c0 = 0; c0 < 72; c0 += 32) {
+    const int c = c0 + lane;
+    const uint32_t own = c < 72 ? P.hist[c] : 0;
+    uint32_t incl = own;
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += o;
+    }
+    if (c < 72) P.hist[c] = carry + incl - own;
+    carry += __shfl_sync(0xffffffffu, incl, 31);
   }
   __syncwarp();
+  for (int p0 = 0; p0 < last; p0 += 32) {
+    const int p = p0 + lane, c = p < last ? P.cls[p] : 71;
+    const uint32_t same = __match_any_sync(0xffffffffu, c), before = same & ((1u << lane) - 1u);
+    const uint32_t at = P.hist[c];
+    __syncwarp();
+    if (p < last) {
+      P.order[at + __popc(before)] = (uint16_t)p;
+      if (!before) P.hist[c] = at + __popc(same);
+    }
+    __syncwarp();
+  }
   auto diff = [&](int p) { return (int64_t)(y[p + 1] - y[p]); };
   auto extremes = [&](int s, int e) { return s == e ? make_longlong2(0, 0) : mm[e]; };  // of segment [s, e]
-  for (int aim = lo; aim <= hi; ++aim) {
+  uint32_t i = 0;  // hist[c] is now where class c ends
+  for (int aim = 0; aim < 71; ++aim) {
+    const uint32_t i1 = P.hist[aim];
     int from = 0;  // segments that end before it have had their turn
-    for (int w = 0; w < words;) {
-      const int e = 32 * w + lane;
-      const bool match = e >= from && e < last && ((P.bits[w] >> lane) & 1u) && P.cls[e] == (uint8_t)aim;
-      if (!__any_sync(0xffffffffu, match)) {
-        ++w;
-        continue;
-      }
+    while (i < i1) {
+      const int e = i + lane < i1 ? P.order[i + lane] : -1;
       // segment c = [s, e] with its right neighbour [e + 1, en]
       int s = 0, en = 0;
       int64_t nmin = 0, nmax = 0;
       bool merge = false;
-      if (match) {
+      if (e >= from && ((P.bits[e >> 5] >> (e & 31)) & 1u)) {
         s = part_prev(P.bits, e) + 1;
         en = part_next(P.bits, e);
         const longlong2 c = extremes(s, e), n = extremes(e + 1, en);
@@ -466,13 +495,14 @@ __device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t
       }
       const uint32_t hit = __ballot_sync(0xffffffffu, merge);
       if (!hit) {
-        ++w;
+        i += 32;
         continue;
       }
       const int f = __ffs((int)hit) - 1;  // the first segment that merges; those before it stay as they are
       int cs = __shfl_sync(0xffffffffu, s, f), ce = __shfl_sync(0xffffffffu, en, f);
       int64_t cmin = __shfl_sync(0xffffffffu, (long long)nmin, f), cmax = __shfl_sync(0xffffffffu, (long long)nmax, f);
-      if (lane == 0) P.bits[w] &= ~(1u << f);
+      const int fe = __shfl_sync(0xffffffffu, e, f);
+      if (lane == 0) P.bits[fe >> 5] &= ~(1u << (fe & 31));
       __syncwarp();
       // grow left (never into the first segment of the block)
       while (cs > 0) {
@@ -510,137 +540,158 @@ __device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t
       if (lane == 0) mm[ce] = make_longlong2(cmin, cmax);
       __syncwarp();
       from = ce + 1;
-      w = from >> 5;
+      i += f + 1;
     }
+    i = i1;
   }
 }
 
-// Fills out[k] for k < count where it holds kNoSize: the size of y[at(k) .. end(k)).
-template <typename At, typename End>
-__device__ __forceinline__ void part_sizes(const uint64_t *y, uint16_t *out, uint32_t count, At at, End end) {
-  const uint32_t lane = threadIdx.x & 31;
-  for (uint32_t k0 = 0; k0 < count; k0 += 32) {
+// Fills out[k] for k < count where it holds kNoSize with the size of y[idx[k] .. idx[k + span]),
+// by the whole CTA; out is complete after the call's last barrier.
+__device__ __forceinline__ void part_sizes(const PartShared &P, uint16_t *out, uint32_t count, uint32_t span) {
+  if (threadIdx.x == 0) P.hist[0] = 0;
+  __syncthreads();
+  for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) {
+    if (out[k] != kNoSize) continue;
+    const uint32_t s = P.idx[k], length = P.idx[k + span] - s;
+    if (length <= kPartLaneMax) out[k] = (uint16_t)lane_size(P.y + s, length);
+    else P.jobs[atomicAdd(&P.hist[0], 1u)] = (uint16_t)k;
+  }
+  __syncthreads();
+  const uint32_t jobs = P.hist[0];
+  for (uint32_t j = threadIdx.x >> 5; j < jobs; j += blockDim.x >> 5) {
+    const uint32_t k = P.jobs[j], s = P.idx[k];
+    const uint32_t z = warp_size(P.y + s, P.idx[k + span] - s);
+    if ((threadIdx.x & 31) == 0) out[k] = (uint16_t)z;
+  }
+  __syncthreads();
+}
+
+// One merge pass by one warp: m segments, their sizes and pair sizes known.  Returns the new
+// number of segments and, in tnew, the sum of their sizes.
+__device__ __forceinline__ uint32_t part_merge_pass(const PartShared &P, uint32_t m, uint32_t len, uint64_t &tnew) {
+  const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+  // From the left: a pair whose size is smaller than its parts' merges and is passed over,
+  // so in a run of such pairs every other one merges, from the run's first on.
+  uint32_t w = 0;      // segments of the new list
+  uint32_t taken = 0;  // 1: the first segment of this group went into the pair before it
+  tnew = 0;
+  // (entries of the list are written no further on than they were read: the group's own
+  // are in registers, and w <= k0; the next group's first pair flag is taken ahead)
+  for (uint32_t k0 = 0; k0 < m; k0 += 32) {
     const uint32_t k = k0 + lane;
-    const bool need = k < count && out[k] == kNoSize;
-    const uint32_t s = need ? at(k) : 0, length = need ? end(k) - s : 0;
-    if (need && length <= kPartLaneMax) out[k] = (uint16_t)lane_size(y + s, length);
-    uint32_t rest = __ballot_sync(0xffffffffu, need && length > kPartLaneMax);
-    while (rest) {
-      const int f = __ffs((int)rest) - 1;
-      rest &= rest - 1;
-      const uint32_t fs = __shfl_sync(0xffffffffu, s, f), fl = __shfl_sync(0xffffffffu, length, f);
-      const uint32_t z = warp_size(y + fs, fl);
-      if ((int)lane == f) out[k] = (uint16_t)z;
-    }
-  }
-  __syncwarp();
-}
-
-// Phase 2: the pairwise merge passes; returns the number of segments, their starts in P.idx.
-__device__ __forceinline__ uint32_t part_merge_pairs(const PartShared &P, uint32_t len, uint32_t bs) {
-  const uint32_t lane = threadIdx.x & 31, last = len - 2;
-  const uint32_t below = (1u << lane) - 1u;
-  // starts: 0 and each end but the last, plus one
-  uint32_t m = 1;
-  if (lane == 0) P.idx[0] = 0;
-  for (uint32_t w = 0; w <= last >> 5; ++w) {
-    uint32_t v = P.bits[w];
-    if (w == last >> 5) v &= ~(1u << (last & 31));
-    if ((v >> lane) & 1u) P.idx[m + __popc(v & below)] = (uint16_t)(32 * w + lane + 1);
-    m += __popc(v);
-  }
-  __syncwarp();
-  if (lane == 0) P.idx[m] = P.idx[m + 1] = (uint16_t)len;  // ends of the last segment and of the last pair
-  for (uint32_t k = lane; k < m; k += 32) {
-    P.sz[k] = kNoSize;
-    P.pc[k] = kNoSize;
-  }
-  __syncwarp();
-  auto start = [&](uint32_t k) -> uint32_t { return P.idx[k]; };
-  part_sizes(P.y, P.sz, m, start, [&](uint32_t k) -> uint32_t { return P.idx[k + 1]; });
-  uint64_t total = 0;
-  for (uint32_t k = lane; k < m; k += 32) total += P.sz[k];
-  total = warp_sum_u64(total);
-  for (;;) {
-    part_sizes(P.y, P.pc, m - 1, start, [&](uint32_t k) -> uint32_t { return P.idx[k + 2]; });
-    // From the left: a pair whose size is smaller than its parts' merges and is passed over,
-    // so in a run of such pairs every other one merges, from the run's first on.
-    uint32_t w = 0;          // segments of the new list
-    uint32_t taken = 0;      // 1: the first segment of this group went into the pair before it
-    uint64_t tnew = 0;
-    // (entries of the list are written no further on than they were read: the group's own
-    // are in registers, and w <= k0; the next group's first pair flag is taken ahead)
-    for (uint32_t k0 = 0; k0 < m; k0 += 32) {
-      const uint32_t k = k0 + lane;
-      const uint32_t z = k < m ? P.sz[k] : 0, q = k + 1 < m ? P.pc[k] : kNoSize;
-      const uint32_t z1 = k + 1 < m ? P.sz[k + 1] : 0, i0 = k < m ? P.idx[k] : 0;
-      const bool want = k + 1 < m && z + z1 > q;
-      uint32_t f = __ballot_sync(0xffffffffu, want) & ~taken;
-      const uint32_t even = 0x55555555u, run0 = f & ~(f << 1);
-      const uint32_t from_even = f & ~(f + (run0 & even));  // the runs that begin at an even place
-      const uint32_t merge = (from_even & even) | ((f & ~from_even) & ~even);
-      const uint32_t gone = (merge << 1) | taken, in = m - k0 >= 32 ? 0xffffffffu : (1u << (m - k0)) - 1u;
-      const uint32_t keep = ~gone & in;
-      // the pair (k, k + 1) stays a pair when neither merges (k + 1's flag may be the next group's)
-      const uint32_t k1 = k0 + 32;
-      uint32_t next_merges = 0;
-      if (!(merge >> 31) && k1 < m) {  // segment k1 is free: does it merge?
-        const uint32_t a = P.sz[k1], b = k1 + 1 < m ? P.sz[k1 + 1] : 0, c = k1 + 1 < m ? P.pc[k1] : kNoSize;
-        next_merges = k1 + 1 < m && a + b > c;
-      }
-      const uint32_t after = (merge >> 1) | (next_merges << 31);  // does segment k + 1 merge
-      __syncwarp();
-      if ((keep >> lane) & 1u) {
-        const uint32_t o = w + __popc(keep & below);
-        const bool mg = (merge >> lane) & 1u;
-        const uint32_t nz = mg ? q : z;
-        P.idx[o] = (uint16_t)i0;
-        P.sz[o] = (uint16_t)nz;
-        P.pc[o] = mg || ((after >> lane) & 1u) ? kNoSize : (uint16_t)q;
-        tnew += nz;
-      }
-      w += __popc(keep);
-      taken = merge >> 31;
-      __syncwarp();
-    }
-    m = w;
-    if (lane == 0) P.idx[m] = P.idx[m + 1] = (uint16_t)len;
+    const uint32_t z = k < m ? P.sz[k] : 0, q = k + 1 < m ? P.pc[k] : kNoSize;
+    const uint32_t z1 = k + 1 < m ? P.sz[k + 1] : 0, i0 = k < m ? P.idx[k] : 0;
+    const bool want = k + 1 < m && z + z1 > q;
+    const uint32_t f = __ballot_sync(0xffffffffu, want) & ~taken;
+    const uint32_t even = 0x55555555u, run0 = f & ~(f << 1);
+    const uint32_t from_even = f & ~(f + (run0 & even));  // the runs that begin at an even place
+    const uint32_t merge = (from_even & even) | ((f & ~from_even) & ~even);
+    const uint32_t gone = (merge << 1) | taken, in = m - k0 >= 32 ? 0xffffffffu : (1u << (m - k0)) - 1u;
+    const uint32_t keep = ~gone & in;
+    // the pair (k, k + 1) stays a pair when neither merges (k + 1's flag may be the next group's)
+    const uint32_t k1 = k0 + 32;
+    uint32_t next_merges = 0;
+    if (!(merge >> 31) && k1 + 1 < m) next_merges = (uint32_t)P.sz[k1] + P.sz[k1 + 1] > P.pc[k1];  // segment k1 is free
+    const uint32_t after = (merge >> 1) | (next_merges << 31);  // does segment k + 1 merge
     __syncwarp();
-    tnew = warp_sum_u64(tnew);
-    const uint64_t decline = total - tnew;  // unsigned, as in the reference
-    total = tnew;
-    const double pct = __ddiv_rn(__dmul_rn(__ull2double_rn(decline), 100.0), __dmul_rn((double)sizeof(uint64_t), (double)bs));
-    if (!(decline > 0) || pct < 0.01) break;
+    if ((keep >> lane) & 1u) {
+      const uint32_t o = w + __popc(keep & below);
+      const bool mg = (merge >> lane) & 1u;
+      const uint32_t nz = mg ? q : z;
+      P.idx[o] = (uint16_t)i0;
+      P.sz[o] = (uint16_t)nz;
+      P.pc[o] = mg || ((after >> lane) & 1u) ? kNoSize : (uint16_t)q;
+      tnew += nz;
+    }
+    w += __popc(keep);
+    taken = merge >> 31;
+    __syncwarp();
   }
-  return m;
+  if (lane == 0) P.idx[w] = P.idx[w + 1] = (uint16_t)len;  // ends of the last segment and of the last pair
+  tnew = warp_sum_u64(tnew);
+  return w;
 }
 
-__global__ void __launch_bounds__(32) partition_warp_kernel(PartitionArgs a) {
+// Phase 2, by the whole CTA: the pairwise merge passes; returns the number of segments, their
+// starts in P.idx.
+__device__ __forceinline__ uint32_t part_merge_pairs(const PartShared &P, uint32_t len, uint32_t bs) {
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, last = len - 2;
+  if (warp == 0) {  // starts: 0 and each end but the last, plus one
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t m = 1;
+    if (lane == 0) P.idx[0] = 0;
+    for (uint32_t w = 0; w <= last >> 5; ++w) {
+      uint32_t v = P.bits[w];
+      if (w == last >> 5) v &= ~(1u << (last & 31));
+      if ((v >> lane) & 1u) P.idx[m + __popc(v & below)] = (uint16_t)(32 * w + lane + 1);
+      m += __popc(v);
+    }
+    __syncwarp();
+    if (lane == 0) {
+      P.idx[m] = P.idx[m + 1] = (uint16_t)len;
+      P.hist[1] = m;
+    }
+  }
+  __syncthreads();
+  uint32_t m = P.hist[1];
+  for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) P.sz[k] = P.pc[k] = kNoSize;
+  part_sizes(P, P.sz, m, 1);
+  uint64_t total = 0;  // warp 0's
+  if (warp == 0) {
+    for (uint32_t k = lane; k < m; k += 32) total += P.sz[k];
+    total = warp_sum_u64(total);
+  }
+  for (;;) {
+    part_sizes(P, P.pc, m - 1, 2);
+    if (warp == 0) {
+      uint64_t tnew;
+      const uint32_t w = part_merge_pass(P, m, len, tnew);
+      const uint64_t decline = total - tnew;  // unsigned, as in the reference
+      total = tnew;
+      const double pct = __ddiv_rn(__dmul_rn(__ull2double_rn(decline), 100.0), __dmul_rn((double)sizeof(uint64_t), (double)bs));
+      if (lane == 0) {
+        P.hist[1] = w;
+        P.hist[2] = !(decline > 0) || pct < 0.01;
+      }
+    }
+    __syncthreads();
+    m = P.hist[1];
+    if (P.hist[2]) return m;
+  }
+}
+
+__global__ void __launch_bounds__(32 * kPartWarps) partition_cta_kernel(PartitionArgs a) {
   extern __shared__ __align__(16) uint8_t part_smem[];
-  const uint32_t lane = threadIdx.x;
+  __shared__ uint32_t ticket;
+  const uint32_t tid = threadIdx.x;
   const PartShared P = part_shared(part_smem, a.bs);
   longlong2 *mm = reinterpret_cast<longlong2 *>(a.segs) + (size_t)blockIdx.x * a.bs;
   for (;;) {
-    uint32_t t = 0;
-    if (lane == 0) t = atomicAdd(a.ticket, 1u);
-    const uint64_t b = __shfl_sync(0xffffffffu, t, 0);
+    __syncthreads();  // the block before has been written out
+    if (tid == 0) ticket = atomicAdd(a.ticket, 1u);
+    if (tid < 72) P.hist[tid] = 0;
+    __syncthreads();
+    const uint64_t b = ticket;
     if (b >= a.nblocks) return;
     const uint64_t B0 = b * a.bs;
     const uint32_t len = (uint32_t)(b == a.nblocks - 1 ? a.n - B0 : a.bs);
     if (len < 2) {  // the reference needs two points per coarse block (it reads array[B0 + 1])
-      if (lane == 0) {
+      if (tid == 0) {
         a.stage[B0] = (uint32_t)B0;
         a.count[b] = 1;
       }
       continue;
     }
-    for (uint32_t i = lane; i < len; i += 32) P.y[i] = __ldg(a.array + B0 + i);
-    __syncwarp();
-    part_merge_classes(P, len, a.overhead, mm);
+    for (uint32_t i = tid; i < len; i += blockDim.x) P.y[i] = __ldg(a.array + B0 + i);
+    __syncthreads();
+    part_classes(P, len);
+    __syncthreads();
+    if (tid < 32) part_merge_classes(P, len, a.overhead, mm);
+    __syncthreads();
     const uint32_t m = part_merge_pairs(P, len, a.bs);
-    for (uint32_t k = lane; k < m; k += 32) a.stage[B0 + k] = (uint32_t)B0 + P.idx[k];
-    if (lane == 0) a.count[b] = m;
-    __syncwarp();
+    for (uint32_t k = tid; k < m; k += blockDim.x) a.stage[B0 + k] = (uint32_t)B0 + P.idx[k];
+    if (tid == 0) a.count[b] = m;
   }
 }
 
@@ -760,20 +811,20 @@ int leco_varlen_partition_device(const uint64_t *d_values, uint64_t n, uint32_t 
   A.ticket = reinterpret_cast<uint32_t *>(w);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(A.ticket, 0, 4, st) != cudaSuccess) return record_error(LECO_ERR_CUDA, "leco_varlen_partition_device: memset");
-  if (bs <= kPartWarpMax) {
+  if (bs <= kPartCtaMax) {
     const uint32_t smem = part_smem_bytes(bs);
     cudaError_t se = cudaSuccess;
     if (smem > 48 * 1024)
-      se = cudaFuncSetAttribute(partition_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      se = cudaFuncSetAttribute(partition_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int dev = 0, sms = 148, per_sm = 1;
     if (se == cudaSuccess) se = cudaGetDevice(&dev);
     if (se == cudaSuccess) se = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (se == cudaSuccess) se = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, partition_warp_kernel, 32, smem);
+    if (se == cudaSuccess) se = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, partition_cta_kernel, 32 * kPartWarps, smem);
     if (se != cudaSuccess)
       return record_error(LECO_ERR_CUDA, std::string("leco_varlen_partition_device: ") + cudaGetErrorString(se));
-    // a warp's scratch (16 bytes a value) lies in its slot's segment list (48 bytes a value): no more warps than slots
+    // a CTA's scratch (16 bytes a value) lies in its slot's segment list (48 bytes a value): no more CTAs than slots
     const uint64_t grid = std::min<uint64_t>(std::min<uint64_t>(nb, slots), (uint64_t)sms * (uint64_t)std::max(per_sm, 1));
-    partition_warp_kernel<<<(unsigned)grid, 32, smem, st>>>(A);
+    partition_cta_kernel<<<(unsigned)grid, 32 * kPartWarps, smem, st>>>(A);
   } else {
     partition_kernel<<<(unsigned)(slots / kPartThreads), kPartThreads, 0, st>>>(A);
   }
