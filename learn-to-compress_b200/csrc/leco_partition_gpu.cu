@@ -298,42 +298,46 @@ __global__ void __launch_bounds__(kPartThreads) partition_kernel(PartitionArgs a
 // first difference D[p] = y[p+1] - y[p]), so a bitmap of the positions where a segment ends
 // is the list; a segment ending at e has the bit class of D[e], D[e+1] and the difference
 // D[e] to its successor, whatever it has absorbed, and starts after the bit before e.  Only
-// the extremes of the differences inside a merged segment are kept, in global memory at
-// its end (single points have none).  The positions are sorted by bit class once, so that a
+// the extremes of the differences inside a merged segment are kept (single points have
+// none), for the first kPartPool of them in shared memory, else in global memory.  The positions are sorted by bit class once, so that a
 // class's turn visits its own positions only, 32 at a time; a position that has been
 // absorbed is skipped.  Phase 2 keeps 16-bit starts, sizes and pair sizes; a pair's size is
 // computed again only when one of the two segments has changed.
 // Bound by latency: phase 1 is one warp's, phase 2 mostly sums of the fits.  Shared memory:
 // 14 bytes a value, eight CTAs per SM for blocks of 2000 values.  10M values, 5000 blocks of
 // 2000, partition and encode: 43.7 ms with a thread per block, 4.47 ms with one warp per
-// block that scanned every class over all positions, 2.59 ms now.
+// block that scanned every class over all positions, 1.86 ms now.
 constexpr uint32_t kPartCtaMax = 8000;   // sizes fit 16 bits, shared memory fits an SM twice
 constexpr uint32_t kPartLaneMax = 48;    // pairs of up to this many values: one lane each
 constexpr uint32_t kPartWarps = 4;
-constexpr uint16_t kNoSize = 0xffffu;
+constexpr uint32_t kPartPool = 192;      // merged segments whose extremes are in shared memory
+constexpr uint16_t kNoSize = 0xffffu, kNoSlot = 0xffffu;
 
 struct PartShared {
   uint64_t *y;
   uint16_t *idx, *sz, *pc;
   uint16_t *order;  // phase 1 (over idx): positions by class
+  uint16_t *slot;   // phase 1 (over pc): a merged segment's place in the pool, at its end
+  longlong2 *pool;  // (min, max) as I (below), two to an entry
   uint8_t *cls;     // phase 1 (over sz)
   uint32_t *bits;   // phase 1: segment ends
-  uint32_t *hist;   // phase 1: [72] where a class's positions end in order; phase 2: [0] long pairs, [1] segments, [2] done
+  uint32_t *hist;   // phase 1: [72] where a class's positions end in order; phase 2: [0] long pairs, [1] segments, [2] sizes missing, [3] done
   uint16_t *jobs;   // phase 2 (over bits): pairs that take a warp
 };
 __host__ __device__ inline uint32_t part_list_bytes(uint32_t bs) { return ((bs + 2) * 2 + 7) / 8 * 8; }
 __host__ __device__ inline uint32_t part_jobs_bytes(uint32_t bs) { return (bs / 32 + 2) * 4 + (bs / kPartLaneMax + 4) * 2 * 2; }
 __host__ __device__ inline uint32_t part_smem_bytes(uint32_t bs) {
-  return bs * 8 + 3 * part_list_bytes(bs) + 72 * 4 + part_jobs_bytes(bs);
+  return kPartPool * 16 + bs * 8 + 3 * part_list_bytes(bs) + 72 * 4 + part_jobs_bytes(bs);
 }
 __device__ __forceinline__ PartShared part_shared(uint8_t *smem, uint32_t bs) {
   const uint32_t list = part_list_bytes(bs);
   PartShared P;
-  P.y = reinterpret_cast<uint64_t *>(smem);
-  uint8_t *p = smem + (size_t)bs * 8;
+  P.pool = reinterpret_cast<longlong2 *>(smem);
+  P.y = reinterpret_cast<uint64_t *>(smem + kPartPool * 16);
+  uint8_t *p = smem + kPartPool * 16 + (size_t)bs * 8;
   P.idx = P.order = reinterpret_cast<uint16_t *>(p);
   P.sz = reinterpret_cast<uint16_t *>(p + list);
-  P.pc = reinterpret_cast<uint16_t *>(p + 2 * list);
+  P.pc = P.slot = reinterpret_cast<uint16_t *>(p + 2 * list);
   P.cls = p + list;
   P.hist = reinterpret_cast<uint32_t *>(p + 3 * list);
   P.bits = P.hist + 72;
@@ -341,12 +345,22 @@ __device__ __forceinline__ PartShared part_shared(uint8_t *smem, uint32_t bs) {
   return P;
 }
 
-// cal_bits with the ceiling of half the difference as an integer where that is exact.
+// cal_bits on integers where that is exact: bits of ceil(d / 2) plus one is the bits of d + 1.
 __device__ __forceinline__ int cal_bits_fast(int64_t mn, int64_t mx) {
   const int64_t diff = (int64_t)((uint64_t)mx - (uint64_t)mn);
   const uint64_t ad = diff < 0 ? 0 - (uint64_t)diff : (uint64_t)diff;
   if (ad >= (1ull << 53)) return cal_bits_d(mn, mx);
-  return ad ? (int)bits64_d((ad + 1) >> 1) + 1 : 0;
+  return ad ? (int)bits64_d(ad + 1) : 0;
+}
+// The same for mn <= mx; I = int32_t: both in (-2^30, 2^30).
+template <typename I>
+__device__ __forceinline__ int span_bits(I mn, I mx) {
+  if constexpr (sizeof(I) == 4) {
+    const uint32_t d = (uint32_t)(mx - mn);
+    return d ? 32 - __clz((int)(d + 1)) : 0;
+  } else {
+    return cal_bits_fast(mn, mx);
+  }
 }
 // The segment end before position e (-1: none) and the one after it (one exists).
 __device__ __forceinline__ int part_prev(const uint32_t *bits, int e) {
@@ -429,6 +443,7 @@ __device__ __noinline__ uint32_t warp_size(const uint64_t *y, uint32_t length) {
 }
 
 // Classes of a coarse block of len >= 2 values, every position a segment; by the whole CTA.
+// hist[71]: nonzero when some difference lies outside (-2^30, 2^30).
 __device__ __forceinline__ void part_classes(const PartShared &P, uint32_t len) {
   const int last = (int)len - 2;  // the last segment's end
   const uint64_t *y = P.y;
@@ -438,19 +453,29 @@ __device__ __forceinline__ void part_classes(const PartShared &P, uint32_t len) 
     P.cls[p] = (uint8_t)c;
     atomicAdd(&P.hist[c], 1u);
   }
+  for (int p = threadIdx.x; p <= last; p += blockDim.x) {
+    const int64_t d = (int64_t)(y[p + 1] - y[p]);
+    if (d <= -(1ll << 30) || d >= 1ll << 30) P.hist[71] = 1;
+  }
   const int words = (last >> 5) + 1;
   for (int w = threadIdx.x; w < words; w += blockDim.x) P.bits[w] = 32 * w + 31 <= last ? 0xffffffffu : (2u << (last & 31)) - 1u;
 }
 
-// Phase 1, by one warp; mm: the merged segments' (min, max) differences, at their ends.
+// Phase 1, by one warp; mm: the (min, max) differences of merged segments that the pool has
+// no place for, at their ends.  I: the type of differences, int32_t when all are small.
+template <typename I>
 __device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t len, int overhead, longlong2 *mm) {
   const int lane = threadIdx.x & 31, last = (int)len - 2;
   const uint64_t *y = P.y;
+  struct Ext {
+    I lo, hi;
+  };
+  Ext *pool = reinterpret_cast<Ext *>(P.pool), *far = reinterpret_cast<Ext *>(mm);
   // positions by class, in order within a class
   uint32_t carry = 0;
   for (int c0 = 0; c0 < 72; c0 += 32) {
     const int c = c0 + lane;
-    const uint32_t own = c < 72 ? P.hist[c] : 0;
+    const uint32_t own = c < 71 ? P.hist[c] : 0;
     uint32_t incl = own;
     for (int d = 1; d < 32; d <<= 1) {
       const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
@@ -471,8 +496,13 @@ __device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t
     }
     __syncwarp();
   }
-  auto diff = [&](int p) { return (int64_t)(y[p + 1] - y[p]); };
-  auto extremes = [&](int s, int e) { return s == e ? make_longlong2(0, 0) : mm[e]; };  // of segment [s, e]
+  auto diff = [&](int p) { return (I)(y[p + 1] - y[p]); };
+  auto extremes = [&](int s, int e) {  // of segment [s, e]
+    if (s == e) return Ext{0, 0};
+    const uint32_t at = P.slot[e];
+    return at == kNoSlot ? far[e] : pool[at];
+  };
+  uint32_t pooled = 0;  // places of the pool handed out; a merge keeps a place of its parts
   uint32_t i = 0;  // hist[c] is now where class c ends
   for (int aim = 0; aim < 71; ++aim) {
     const uint32_t i1 = P.hist[aim];
@@ -481,17 +511,17 @@ __device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t
       const int e = i + lane < i1 ? P.order[i + lane] : -1;
       // segment c = [s, e] with its right neighbour [e + 1, en]
       int s = 0, en = 0;
-      int64_t nmin = 0, nmax = 0;
+      Ext x{0, 0};
       bool merge = false;
       if (e >= from && ((P.bits[e >> 5] >> (e & 31)) & 1u)) {
         s = part_prev(P.bits, e) + 1;
         en = part_next(P.bits, e);
-        const longlong2 c = extremes(s, e), n = extremes(e + 1, en);
-        const int64_t d = diff(e);
-        nmax = max(max((int64_t)c.y, (int64_t)n.y), d);
-        nmin = min(min((int64_t)c.x, (int64_t)n.x), d);
-        const int origin = (e + 1 - s) * cal_bits_fast(c.x, c.y) + (en - e) * cal_bits_fast(n.x, n.y);
-        merge = cal_bits_fast(nmin, nmax) * (en - s + 1) - origin < overhead;
+        const Ext c = extremes(s, e), n = extremes(e + 1, en);
+        const I d = diff(e);
+        x.hi = max(max(c.hi, n.hi), d);
+        x.lo = min(min(c.lo, n.lo), d);
+        const int origin = (e + 1 - s) * span_bits(c.lo, c.hi) + (en - e) * span_bits(n.lo, n.hi);
+        merge = span_bits(x.lo, x.hi) * (en - s + 1) - origin < overhead;
       }
       const uint32_t hit = __ballot_sync(0xffffffffu, merge);
       if (!hit) {
@@ -499,45 +529,63 @@ __device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t
         continue;
       }
       const int f = __ffs((int)hit) - 1;  // the first segment that merges; those before it stay as they are
+      uint32_t place = kNoSlot;  // of the merged segment
+      auto inherit = [&](int a, int b) {  // segment [a, b] is absorbed
+        if (a != b && place == kNoSlot) place = P.slot[b];
+      };
       int cs = __shfl_sync(0xffffffffu, s, f), ce = __shfl_sync(0xffffffffu, en, f);
-      int64_t cmin = __shfl_sync(0xffffffffu, (long long)nmin, f), cmax = __shfl_sync(0xffffffffu, (long long)nmax, f);
+      x.lo = __shfl_sync(0xffffffffu, x.lo, f);
+      x.hi = __shfl_sync(0xffffffffu, x.hi, f);
       const int fe = __shfl_sync(0xffffffffu, e, f);
+      inherit(cs, fe);
+      inherit(fe + 1, ce);
+      __syncwarp();  // every lane has read the bits
       if (lane == 0) P.bits[fe >> 5] &= ~(1u << (fe & 31));
       __syncwarp();
+      int width = span_bits(x.lo, x.hi);
       // grow left (never into the first segment of the block)
       while (cs > 0) {
         const int pe = cs - 1, ps = part_prev(P.bits, pe) + 1;
         if (ps == 0) break;
-        const longlong2 p = extremes(ps, pe);
-        const int64_t d = diff(pe);
-        const int64_t lmax = max(max((int64_t)p.y, cmax), d), lmin = min(min((int64_t)p.x, cmin), d);
-        const int oc = (cs - ps) * cal_bits_fast(p.x, p.y) + (ce - cs + 1) * cal_bits_fast(cmin, cmax);
-        if (!(cal_bits_fast(lmin, lmax) * (ce - ps + 1) - oc < overhead)) break;
-        __syncwarp();  // every lane has read the bits
+        const Ext p = extremes(ps, pe);
+        const I d = diff(pe);
+        const Ext g{min(min(p.lo, x.lo), d), max(max(p.hi, x.hi), d)};
+        const int gw = span_bits(g.lo, g.hi);
+        const int oc = (cs - ps) * span_bits(p.lo, p.hi) + (ce - cs + 1) * width;
+        if (!(gw * (ce - ps + 1) - oc < overhead)) break;
+        inherit(ps, pe);
+        __syncwarp();
         if (lane == 0) P.bits[pe >> 5] &= ~(1u << (pe & 31));
         __syncwarp();
         cs = ps;
-        cmin = lmin;
-        cmax = lmax;
+        x = g;
+        width = gw;
       }
       // grow right (never into the last segment of the block)
       while (ce < last) {
         const int ne = part_next(P.bits, ce);
         if (ne == last) break;
-        const longlong2 n = extremes(ce + 1, ne);
-        const int64_t d = diff(ce);
-        const int64_t rmax = max(max((int64_t)n.y, cmax), d), rmin = min(min((int64_t)n.x, cmin), d);
-        const int oc = (ne - ce) * cal_bits_fast(n.x, n.y) + (ce + 1 - cs) * cal_bits_fast(cmin, cmax);
-        if (!(cal_bits_fast(rmin, rmax) * (ne - cs + 1) - oc < overhead)) break;
+        const Ext n = extremes(ce + 1, ne);
+        const I d = diff(ce);
+        const Ext g{min(min(n.lo, x.lo), d), max(max(n.hi, x.hi), d)};
+        const int gw = span_bits(g.lo, g.hi);
+        const int oc = (ne - ce) * span_bits(n.lo, n.hi) + (ce + 1 - cs) * width;
+        if (!(gw * (ne - cs + 1) - oc < overhead)) break;
+        inherit(ce + 1, ne);
         __syncwarp();
         if (lane == 0) P.bits[ce >> 5] &= ~(1u << (ce & 31));
         __syncwarp();
         ce = ne;
-        cmin = rmin;
-        cmax = rmax;
+        x = g;
+        width = gw;
       }
+      if (place == kNoSlot && pooled < kPartPool) place = pooled++;
       __syncwarp();
-      if (lane == 0) mm[ce] = make_longlong2(cmin, cmax);
+      if (lane == 0) {
+        P.slot[ce] = (uint16_t)place;
+        if (place != kNoSlot) pool[place] = x;
+        else far[ce] = x;
+      }
       __syncwarp();
       from = ce + 1;
       i += f + 1;
@@ -546,13 +594,15 @@ __device__ __forceinline__ void part_merge_classes(const PartShared &P, uint32_t
   }
 }
 
-// Fills out[k] for k < count where it holds kNoSize with the size of y[idx[k] .. idx[k + span]),
-// by the whole CTA; out is complete after the call's last barrier.
-__device__ __forceinline__ void part_sizes(const PartShared &P, uint16_t *out, uint32_t count, uint32_t span) {
+// Fills out[k] for k < count where it holds kNoSize and take(k) with the size of
+// y[idx[k] .. idx[k + span]), by the whole CTA; out is complete after the call's last barrier.
+template <typename Take>
+__device__ __forceinline__ void part_sizes(const PartShared &P, uint16_t *out, uint32_t first, uint32_t step, uint32_t count,
+                                           uint32_t span, Take take) {
   if (threadIdx.x == 0) P.hist[0] = 0;
   __syncthreads();
-  for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) {
-    if (out[k] != kNoSize) continue;
+  for (uint32_t k = first + step * threadIdx.x; k < count; k += step * blockDim.x) {
+    if (out[k] != kNoSize || !take(k)) continue;
     const uint32_t s = P.idx[k], length = P.idx[k + span] - s;
     if (length <= kPartLaneMax) out[k] = (uint16_t)lane_size(P.y + s, length);
     else P.jobs[atomicAdd(&P.hist[0], 1u)] = (uint16_t)k;
@@ -566,13 +616,34 @@ __device__ __forceinline__ void part_sizes(const PartShared &P, uint16_t *out, u
   }
   __syncthreads();
 }
+// The groups of 32 pairs of a pass, from the left: a pair whose size is smaller than its
+// parts' merges and is passed over, so in a run of such pairs every other one merges, from
+// the run's first on.  want: the pairs that would merge; taken: 1 when the group's first
+// segment went into the pair before it.  Returns the pairs that merge.
+__device__ __forceinline__ uint32_t part_merging(uint32_t want, uint32_t taken) {
+  const uint32_t f = want & ~taken, even = 0x55555555u, run0 = f & ~(f << 1);
+  const uint32_t from_even = f & ~(f + (run0 & even));  // the runs that begin at an even place
+  return (from_even & even) | ((f & ~from_even) & ~even);
+}
+// True when a pass would come to a pair whose size is not known (one warp).
+__device__ __forceinline__ bool part_pairs_missing(const PartShared &P, uint32_t m) {
+  const uint32_t lane = threadIdx.x & 31;
+  uint32_t taken = 0;
+  for (uint32_t k0 = 0; k0 + 1 < m; k0 += 32) {
+    const uint32_t k = k0 + lane;
+    const uint32_t q = k + 1 < m ? P.pc[k] : kNoSize, z = k + 1 < m ? (uint32_t)P.sz[k] + P.sz[k + 1] : 0;
+    const uint32_t merge = part_merging(__ballot_sync(0xffffffffu, z > q), taken);
+    const uint32_t unknown = __ballot_sync(0xffffffffu, k + 1 < m && q == kNoSize);
+    if (unknown & ~((merge << 1) | taken)) return true;
+    taken = merge >> 31;
+  }
+  return false;
+}
 
-// One merge pass by one warp: m segments, their sizes and pair sizes known.  Returns the new
+// One merge pass by one warp: m segments, their sizes and the pair sizes it comes to known.  Returns the new
 // number of segments and, in tnew, the sum of their sizes.
 __device__ __forceinline__ uint32_t part_merge_pass(const PartShared &P, uint32_t m, uint32_t len, uint64_t &tnew) {
   const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
-  // From the left: a pair whose size is smaller than its parts' merges and is passed over,
-  // so in a run of such pairs every other one merges, from the run's first on.
   uint32_t w = 0;      // segments of the new list
   uint32_t taken = 0;  // 1: the first segment of this group went into the pair before it
   tnew = 0;
@@ -583,10 +654,7 @@ __device__ __forceinline__ uint32_t part_merge_pass(const PartShared &P, uint32_
     const uint32_t z = k < m ? P.sz[k] : 0, q = k + 1 < m ? P.pc[k] : kNoSize;
     const uint32_t z1 = k + 1 < m ? P.sz[k + 1] : 0, i0 = k < m ? P.idx[k] : 0;
     const bool want = k + 1 < m && z + z1 > q;
-    const uint32_t f = __ballot_sync(0xffffffffu, want) & ~taken;
-    const uint32_t even = 0x55555555u, run0 = f & ~(f << 1);
-    const uint32_t from_even = f & ~(f + (run0 & even));  // the runs that begin at an even place
-    const uint32_t merge = (from_even & even) | ((f & ~from_even) & ~even);
+    const uint32_t merge = part_merging(__ballot_sync(0xffffffffu, want), taken);
     const uint32_t gone = (merge << 1) | taken, in = m - k0 >= 32 ? 0xffffffffu : (1u << (m - k0)) - 1u;
     const uint32_t keep = ~gone & in;
     // the pair (k, k + 1) stays a pair when neither merges (k + 1's flag may be the next group's)
@@ -636,14 +704,24 @@ __device__ __forceinline__ uint32_t part_merge_pairs(const PartShared &P, uint32
   __syncthreads();
   uint32_t m = P.hist[1];
   for (uint32_t k = threadIdx.x; k < m; k += blockDim.x) P.sz[k] = P.pc[k] = kNoSize;
-  part_sizes(P, P.sz, m, 1);
+  part_sizes(P, P.sz, 0, 1, m, 1, [](uint32_t) { return true; });
   uint64_t total = 0;  // warp 0's
   if (warp == 0) {
     for (uint32_t k = lane; k < m; k += 32) total += P.sz[k];
     total = warp_sum_u64(total);
   }
   for (;;) {
-    part_sizes(P, P.pc, m - 1, 2);
+    // Most pairs merge while segments are short, and a pair that merges keeps the next one from
+    // being looked at: every other pair first, then those after a pair that does not merge,
+    // and the rest only if the pass would come to one of them.
+    part_sizes(P, P.pc, 0, 2, m - 1, 2, [](uint32_t) { return true; });
+    part_sizes(P, P.pc, 1, 2, m - 1, 2, [&](uint32_t k) { return (uint32_t)P.sz[k - 1] + P.sz[k] <= P.pc[k - 1]; });
+    if (warp == 0) {
+      const bool missing = part_pairs_missing(P, m);
+      if (lane == 0) P.hist[2] = missing;
+    }
+    __syncthreads();
+    if (P.hist[2]) part_sizes(P, P.pc, 0, 1, m - 1, 2, [](uint32_t) { return true; });
     if (warp == 0) {
       uint64_t tnew;
       const uint32_t w = part_merge_pass(P, m, len, tnew);
@@ -652,12 +730,12 @@ __device__ __forceinline__ uint32_t part_merge_pairs(const PartShared &P, uint32
       const double pct = __ddiv_rn(__dmul_rn(__ull2double_rn(decline), 100.0), __dmul_rn((double)sizeof(uint64_t), (double)bs));
       if (lane == 0) {
         P.hist[1] = w;
-        P.hist[2] = !(decline > 0) || pct < 0.01;
+        P.hist[3] = !(decline > 0) || pct < 0.01;
       }
     }
     __syncthreads();
     m = P.hist[1];
-    if (P.hist[2]) return m;
+    if (P.hist[3]) return m;
   }
 }
 
@@ -687,7 +765,10 @@ __global__ void __launch_bounds__(32 * kPartWarps) partition_cta_kernel(Partitio
     __syncthreads();
     part_classes(P, len);
     __syncthreads();
-    if (tid < 32) part_merge_classes(P, len, a.overhead, mm);
+    if (tid < 32) {
+      if (P.hist[71]) part_merge_classes<int64_t>(P, len, a.overhead, mm);
+      else part_merge_classes<int32_t>(P, len, a.overhead, mm);
+    }
     __syncthreads();
     const uint32_t m = part_merge_pairs(P, len, a.bs);
     for (uint32_t k = tid; k < m; k += blockDim.x) a.stage[B0 + k] = (uint32_t)B0 + P.idx[k];
