@@ -392,9 +392,12 @@ def _torch():
 
 
 def _stream_ptr(stream=None):
+    if stream is not None:
+        return _P(stream.cuda_stream)
     torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return _P(s.cuda_stream)
+    # the current device's current stream as torch.cuda.current_stream() gives it, without the
+    # stream object it builds on each call (0.5 against 3.5 us, of ~20 us for a small encode)
+    return _P(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def _tptr(t):

@@ -359,13 +359,10 @@ static void run_decode(const DecodeLaunch &L, cudaStream_t st) {
     else decode_kernel<T, CODEC><<<(unsigned)nblk, 256, 0, st>>>(L);
     return;
   }
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int smem = 2 * kStageBuf + 64;  // +64: field reads may run a few bytes past a full buffer
-  cudaFuncSetAttribute(decode_staged_kernel<T, CODEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_staged_kernel<T, CODEC>, 256, smem);
-  const uint64_t grid = umin64(nblk, (uint64_t)sms * (uint64_t)(per_sm > 0 ? per_sm : 1));
+  const LaunchInfo i = launch_info<decode_staged_kernel<T, CODEC, false>>(256, smem);
+  if (i.error != cudaSuccess) return;  // the caller reports it
+  const uint64_t grid = umin64(nblk, (uint64_t)i.sms * (uint64_t)i.per_sm);
   decode_staged_kernel<T, CODEC><<<(unsigned)grid, 256, smem, st>>>(L, kStageBuf);
 }
 int launch_decode(int codec, int s, const DecodeLaunch &L, cudaStream_t st) { LECO_DISPATCH(codec, s, run_decode, L, st); }
@@ -380,13 +377,10 @@ static void run_sum(const DecodeLaunch &L, uint64_t *d_sum, cudaStream_t st) {
     sum_kernel<T, CODEC><<<(unsigned)nb, 256, 0, st>>>(L, d_sum);
     return;
   }
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int smem = 2 * kStageBuf + 64;
-  cudaFuncSetAttribute(decode_staged_kernel<T, CODEC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, decode_staged_kernel<T, CODEC, true>, 256, smem);
-  const uint64_t grid = umin64(nb, (uint64_t)sms * (uint64_t)(per_sm > 0 ? per_sm : 1));
+  const LaunchInfo i = launch_info<decode_staged_kernel<T, CODEC, true>>(256, smem);
+  if (i.error != cudaSuccess) return;  // the caller reports it
+  const uint64_t grid = umin64(nb, (uint64_t)i.sms * (uint64_t)i.per_sm);
   decode_staged_kernel<T, CODEC, true><<<(unsigned)grid, 256, smem, st>>>(L, kStageBuf, d_sum);
 }
 int launch_sum(int codec, int s, const DecodeLaunch &L, uint64_t *d_sum, cudaStream_t st) {
@@ -396,16 +390,17 @@ int launch_sum(int codec, int s, const DecodeLaunch &L, uint64_t *d_sum, cudaStr
 template <typename T, int CODEC>
 static void run_gather(const GatherLaunch &L, cudaStream_t st) {
   if (!L.m) return;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (CODEC == kDelta) {  // one warp per lookup at a time
-    const unsigned grid = (unsigned)umin64((L.m + 7) / 8, (uint64_t)sms * 8);
+  if constexpr (CODEC == kDelta) {  // one warp per lookup at a time
+    const LaunchInfo i = launch_info<gather_delta_kernel<T>>(256, 0);
+    if (i.error != cudaSuccess) return;  // the caller reports it
+    const unsigned grid = (unsigned)umin64((L.m + 7) / 8, (uint64_t)i.sms * 8);
     gather_delta_kernel<T><<<grid, 256, 0, st>>>(L);
     return;
   }
+  const LaunchInfo i = launch_info<gather_kernel<T, CODEC>>(256, 0);
+  if (i.error != cudaSuccess) return;  // the caller reports it
   const uint64_t need = (L.m + 4 * 256 - 1) / (4 * 256);  // 4 lookups in flight per thread
-  const unsigned grid = (unsigned)umin64(need, (uint64_t)sms * 8);
+  const unsigned grid = (unsigned)umin64(need, (uint64_t)i.sms * 8);
   gather_kernel<T, CODEC><<<grid, 256, 0, st>>>(L);
 }
 int launch_gather(int codec, int s, const GatherLaunch &L, cudaStream_t st) { LECO_DISPATCH(codec, s, run_gather, L, st); }

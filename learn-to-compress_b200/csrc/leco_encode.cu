@@ -265,7 +265,7 @@ int launch_encode(int codec, int s, const EncodeLaunch &L, cudaStream_t st) {
     }
     return s == 4 ? launch_rows_u32(codec, a, ref, st) : launch_rows_u64(codec, a, ref, st);
   }
-  if (s != 4) return -1;
+  if (s != 4) return 1;
   if (L.seq_models) {  // the legacy codec fits as LINEAR does
     launch_seq_fit<uint32_t, kLinear>(L, st);
     a.seq_models = L.seq_models;

@@ -1,5 +1,6 @@
 // leco_internal.h -- declarations shared by the library's translation units.
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <cuda_runtime.h>
@@ -76,6 +77,35 @@ int launch_gather(int codec, int s, const GatherLaunch &L, cudaStream_t st);
 int launch_sum(int codec, int s, const DecodeLaunch &L, uint64_t *d_sum, cudaStream_t st);
 int launch_build_dir(int codec, int s, const uint8_t *payload, const uint64_t *offsets, uint64_t n, uint32_t bs,
                      leco_dir_entry *dir, uint32_t *error, cudaStream_t st);
+
+// What a launch needs to know about kernel K on the current device: its SMs and how many
+// CTAs of `threads` threads and `smem` bytes of dynamic shared memory an SM holds (the same
+// for every call with this K).  Asked of the runtime once per device, the opt-in to more than
+// 48 KB with it: the three queries took about as long as a launch.
+struct LaunchInfo {
+  cudaError_t error;
+  int sms, per_sm;
+};
+template <auto K>
+inline LaunchInfo launch_info(int threads, int smem) {
+  static std::atomic<uint64_t> known[64];  // sms << 32 | per_sm; 0: not asked yet
+  int dev = 0;
+  LaunchInfo r{cudaGetDevice(&dev), 0, 0};
+  if (r.error != cudaSuccess) return r;
+  const bool keep = dev >= 0 && dev < 64;
+  const uint64_t v = keep ? known[dev].load(std::memory_order_acquire) : 0;
+  if (v) {
+    r.sms = (int)(v >> 32);
+    r.per_sm = (int)(uint32_t)v;
+    return r;
+  }
+  if (smem > 48 * 1024) r.error = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (r.error == cudaSuccess) r.error = cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, dev);
+  if (r.error == cudaSuccess) r.error = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.per_sm, K, threads, (size_t)smem);
+  if (r.error == cudaSuccess && r.per_sm < 1) r.per_sm = 1;
+  if (r.error == cudaSuccess && keep) known[dev].store(((uint64_t)r.sms << 32) | (uint32_t)r.per_sm, std::memory_order_release);
+  return r;
+}
 
 // Reference X sums of polynomial_regression_iter: X[k] = sum_{j<N} j^k as a
 // sequential FP64 loop (polynomial_regression_internals.hpp:111-116), x^k built

@@ -30,10 +30,9 @@ template <typename T, int CODEC, int NT, uint32_t RT>
 int launch_rows_nt(const EncodeArgs &a, uint32_t R, bool ref, cudaStream_t st) {
   const uint64_t nb_item = NT / R, items = (a.nb + nb_item - 1) / nb_item;
   const uint32_t smem = rows_layout(NT, R, sizeof(T), rows_sums(CODEC)).total;
-  if (smem > 48 * 1024) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(encode_rows_kernel<T, CODEC, NT, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return -(int)e;
+  if (smem > 48 * 1024) {  // (R is fixed in these kernels, so smem is)
+    const LaunchInfo i = launch_info<encode_rows_kernel<T, CODEC, NT, RT>>(NT, (int)smem);
+    if (i.error != cudaSuccess) return -(int)i.error;
   }
   encode_rows_kernel<T, CODEC, NT, RT><<<(unsigned)(items > 1 ? items + 1 : 1), NT, smem, st>>>(a, R, (uint32_t)items, ref);
   return 0;

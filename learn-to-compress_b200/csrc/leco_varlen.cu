@@ -434,14 +434,11 @@ template <bool SUM>
 static cudaError_t launch_varlen_staged(const uint8_t *payload, const uint64_t *offsets, const uint64_t *starts,
                                         uint64_t nseg, uint64_t n, uint64_t *out, uint32_t *err, uint64_t *d_sum,
                                         cudaStream_t st) {
-  int dev = 0, sms = 148, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int smem = (int)(2 * kVarStageBytes);
-  cudaFuncSetAttribute(varlen_decode_kernel<SUM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, varlen_decode_kernel<SUM>, 256, smem);
+  const LaunchInfo i = launch_info<varlen_decode_kernel<SUM>>(256, smem);
+  if (i.error != cudaSuccess) return i.error;
   const uint64_t nitems = (nseg + kVarGroup - 1) / kVarGroup;
-  const unsigned grid = (unsigned)umin64(nitems, (uint64_t)sms * (uint64_t)(per_sm > 0 ? per_sm : 1));
+  const unsigned grid = (unsigned)umin64(nitems, (uint64_t)i.sms * (uint64_t)i.per_sm);
   varlen_decode_kernel<SUM><<<grid, 256, smem, st>>>(payload, offsets, starts, nseg, n, out, kVarStageBytes, err, d_sum);
   return cudaGetLastError();
 }
@@ -574,10 +571,9 @@ int leco_varlen_gather(const uint8_t *d_payload, const uint64_t *d_offsets, cons
   uint32_t *err = nullptr;
   int rc = leco::device_error_word(&err);
   if (rc) return rc;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const unsigned grid = (unsigned)umin64((m + 256 * kVarQ - 1) / (256 * kVarQ), (uint64_t)sms * 4);
+  const LaunchInfo i = launch_info<varlen_gather_kernel>(256, 0);
+  if (i.error != cudaSuccess) return verr(LECO_ERR_CUDA, std::string("leco_varlen_gather: ") + cudaGetErrorString(i.error));
+  const unsigned grid = (unsigned)umin64((m + 256 * kVarQ - 1) / (256 * kVarQ), (uint64_t)i.sms * 4);
   varlen_gather_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(d_payload, d_offsets, d_starts, nseg, n,
                                                                                 d_idx, m, d_out, err);
   cudaError_t e = cudaGetLastError();
