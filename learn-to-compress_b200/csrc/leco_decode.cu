@@ -210,6 +210,209 @@ __global__ void __launch_bounds__(256) decode_staged_kernel(DecodeLaunch a, uint
   }
 }
 
+// ---- Delta decode, staged ----------------------------------------------------------
+// The NV differences of a span whose first field starts `sh` bits into word w[0] of a staged
+// body: v[j] = the sum of the differences before value j, returns the sum of all.  Width L at
+// compile time: the span's words are read once, each field is a shift or two.
+template <typename I, int L, int NV>
+__device__ __forceinline__ I delta_span(const uint32_t *w, uint32_t sh, I (&v)[NV]) {
+  constexpr int NW = (NV * L + 31) / 32;
+  uint32_t x[NW + 1];
+  uint32_t last = w[0];
+#pragma unroll
+  for (int q = 0; q < NW; ++q) {
+    const uint32_t next = w[q + 1];
+    x[q] = __funnelshift_r(last, next, sh);
+    last = next;
+  }
+  x[NW] = 0;
+  I acc = 0;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    constexpr uint32_t m1 = L > 1 ? (1u << (L - 1)) - 1u : 0u;
+    const int p = j * L, q = p >> 5, s = p & 31;
+    const uint32_t f = s + L <= 32 ? x[q] >> s : __funnelshift_r(x[q], x[q + 1], s);
+    const uint32_t up = (uint32_t)((int32_t)(f << (32 - L)) >> 31);  // all ones: + magnitude
+    v[j] = acc;
+    acc += (I)(int32_t)(((f & m1) ^ ~up) + up + 1u);
+  }
+  return acc;
+}
+// NS spans of NV values each, `step` bits apart: their sums before each value and in all.
+template <typename I, int L, int NS, int NV>
+__device__ __forceinline__ void delta_spans(const uint32_t *words, uint32_t bit, uint32_t step, uint32_t have, I (&v)[NS][NV], I (&tot)[NS]) {
+#pragma unroll
+  for (int s = 0; s < NS; ++s) {
+    const uint32_t at = bit + s * step;
+    if ((uint32_t)s < have) {
+      tot[s] = delta_span<I, L, NV>(words + (at >> 5), at & 31, v[s]);
+    } else {
+      tot[s] = 0;
+#pragma unroll
+      for (int j = 0; j < NV; ++j) v[s][j] = 0;
+    }
+  }
+}
+template <typename I, int NS, int NV>
+__device__ __forceinline__ void delta_spans_any(uint32_t l, const uint32_t *words, uint32_t bit, uint32_t step, uint32_t have,
+                                                I (&v)[NS][NV], I (&tot)[NS]) {
+  switch (l) {
+#define LECO_SPAN_CASE(L) \
+  case L: delta_spans<I, L, NS, NV>(words, bit, step, have, v, tot); return;
+    LECO_SPAN_CASE(1) LECO_SPAN_CASE(2) LECO_SPAN_CASE(3) LECO_SPAN_CASE(4) LECO_SPAN_CASE(5) LECO_SPAN_CASE(6)
+    LECO_SPAN_CASE(7) LECO_SPAN_CASE(8) LECO_SPAN_CASE(9) LECO_SPAN_CASE(10) LECO_SPAN_CASE(11) LECO_SPAN_CASE(12)
+    LECO_SPAN_CASE(13) LECO_SPAN_CASE(14) LECO_SPAN_CASE(15) LECO_SPAN_CASE(16) LECO_SPAN_CASE(17) LECO_SPAN_CASE(18)
+    LECO_SPAN_CASE(19) LECO_SPAN_CASE(20) LECO_SPAN_CASE(21) LECO_SPAN_CASE(22) LECO_SPAN_CASE(23) LECO_SPAN_CASE(24)
+    LECO_SPAN_CASE(25) LECO_SPAN_CASE(26) LECO_SPAN_CASE(27) LECO_SPAN_CASE(28) LECO_SPAN_CASE(29) LECO_SPAN_CASE(30)
+    LECO_SPAN_CASE(31) LECO_SPAN_CASE(32)
+#undef LECO_SPAN_CASE
+    default: delta_spans<I, 1, NS, NV>(words, bit, step, 0, v, tot);  // width 0: no differences
+  }
+}
+// Decodes a staged Delta block of len >= 2 values and fields of l <= 32 bits with the whole
+// CTA (256 threads): a warp takes 512 consecutive values, a lane NS spans of NV of them, span
+// s the lane-th of the warp's s-th 32 * NV values -- a store instruction of the warp then
+// covers 32 * NV values without gaps, in 64-byte pieces (with one span of 16 values a lane its
+// 32-byte stores were 128 bytes apart, one line each: 140 us for 60M u64 values).  One tile,
+// and one barrier, for 4096 values.  wt: [2][8] warp totals.  I: int32_t when no sum of the
+// block's differences leaves 32 bits.  Spans past the block's end are not read, and what the
+// last one reads past its end reaches no value that is stored.
+template <typename T, typename I>
+__device__ __forceinline__ void delta_block_staged(const uint32_t *words32, uint32_t body_bit, uint32_t l, uint64_t x0, uint32_t len,
+                                                   T *out, uint64_t *wt) {
+  using A = typename std::conditional<sizeof(T) == 8, uint64_t, uint32_t>::type;  // arithmetic mod 2^(8S)
+  constexpr int NV = 8, NS = 2;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool wide_stores = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+  A carry = (A)x0;
+  for (uint32_t t0 = 0; t0 < len; t0 += 4096) {
+    const uint32_t k0 = t0 + warp * 512 + lane * NV;  // span s starts at k0 + s * 256
+    I v[NS][NV], tot[NS], incl[NS];
+    uint32_t have = 0;
+#pragma unroll
+    for (int s = 0; s < NS; ++s) have += k0 + s * 256 < len;
+    delta_spans_any<I, NS, NV>(l, words32, body_bit + k0 * l, 256 * l, have, v, tot);
+#pragma unroll
+    for (int s = 0; s < NS; ++s) incl[s] = tot[s];
+#pragma unroll
+    for (uint32_t o = 1; o < 32; o <<= 1) {
+#pragma unroll
+      for (int s = 0; s < NS; ++s) {
+        const I y = __shfl_up_sync(0xffffffffu, incl[s], o);
+        if (lane >= o) incl[s] += y;
+      }
+    }
+#pragma unroll
+    for (int s = 1; s < NS; ++s) incl[s] += __shfl_sync(0xffffffffu, incl[s - 1], 31);
+    // the two halves of the totals alternate, so one barrier a tile is enough
+    uint64_t *half = wt + 8 * ((t0 >> 12) & 1);
+    if (lane == 31) half[warp] = (uint64_t)(int64_t)incl[NS - 1];
+    __syncthreads();
+    A before = carry;
+#pragma unroll
+    for (uint32_t w = 0; w < 8; ++w) {
+      const A t = (A)half[w];
+      carry += t;
+      if (w < warp) before += t;
+    }
+#pragma unroll
+    for (int s = 0; s < NS; ++s) {
+      const A first = before + (A)(incl[s] - tot[s]);
+      const uint32_t k = k0 + s * 256;
+      if (k + NV <= len && wide_stores) {
+        uint64_t z[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) z[j] = (uint64_t)(A)(first + (A)v[s][j]);
+        store_vals32<T, NV>(out, k, z);
+      } else {
+#pragma unroll
+        for (int j = 0; j < NV; ++j)
+          if (k + j < len) out[k + j] = (T)(first + (A)v[s][j]);
+      }
+    }
+  }
+}
+
+// Persistent Delta decode of a whole column, staged as decode_staged_kernel stages it.  A
+// CTA's threads leave an iteration together, with the next block's image landed: the barrier
+// that frees the buffer says so too, so a block of 4096 values has two barriers, not three.
+// 60M u64 values (0.58 GB, 91 us at the copy rate): 184 us with eight values per thread and
+// fields addressed one by one (67 instructions a value), 107 us now.
+template <typename T>
+__global__ void __launch_bounds__(256, 4) decode_delta_kernel(DecodeLaunch a, uint32_t bufcap) {
+  constexpr int S = sizeof(T);
+  extern __shared__ __align__(128) uint8_t stage[];
+  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ StageMeta meta[2];
+  __shared__ uint64_t wt[16];
+  const uint32_t tid = threadIdx.x;
+  const uint64_t nblk = (a.n + a.bs - 1) / a.bs;
+  if (tid == 0) {
+    mbar_init(&bar[0], 1);
+    mbar_init(&bar[1], 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  auto issue = [&](uint64_t b, int which) {  // thread 0 only
+    const uint64_t o0 = __ldg(a.offsets + b), o1 = __ldg(a.offsets + b + 1);
+    const uint64_t g0 = o0 & ~15ull, g1 = (o1 + 8 + 15) & ~15ull;  // +8: the field reads touch one word past the body
+    const uint64_t bytes = g1 - g0;
+    StageMeta m;
+    m.gbase = g0;
+    m.hoff = (uint32_t)(o0 - g0);
+    m.direct = bytes > bufcap;
+    meta[which] = m;
+    if (!m.direct) {
+      mbar_arrive_tx(&bar[which], (uint32_t)bytes);
+      bulk_g2s(stage + (size_t)which * bufcap, a.payload + g0, (uint32_t)bytes, &bar[which]);
+    } else {
+      mbar_arrive(&bar[which]);
+    }
+  };
+  uint64_t blk = blockIdx.x;
+  if (blk >= nblk) return;
+  uint32_t ph[2] = {0, 0};
+  if (tid == 0) issue(blk, 0);
+  // A wait that gave up in any thread ends the CTA's work in all of them together.
+  bool ok = mbar_wait_bounded(&bar[0], 0);
+  ph[0] = 1;
+  if (__syncthreads_or(!ok)) {
+    if (tid == 0) atomicOr(a.error, kErrTimeout);
+    return;
+  }
+  T *outp = reinterpret_cast<T *>(a.out);
+  for (int cur = 0;; cur ^= 1) {
+    const uint64_t nxt = blk + gridDim.x;
+    const bool has_next = nxt < nblk;
+    if (tid == 0 && has_next) issue(nxt, cur ^ 1);
+    const StageMeta m = meta[cur];
+    const uint8_t *sb = stage + (size_t)cur * bufcap;
+    const uint32_t l = sb[m.hoff];
+    const uint64_t base = blk * a.bs;
+    const uint32_t len = (uint32_t)umin64(a.bs, a.n - base);
+    if (m.direct || l > 32 || l == 8u * S || len < 2) {
+      decode_block<T, kDelta>(a, blk);
+    } else {
+      uint64_t x0 = 0;
+#pragma unroll
+      for (int j = 0; j < S; ++j) x0 |= (uint64_t)sb[m.hoff + 1 + j] << (8 * j);
+      const uint32_t *w32 = reinterpret_cast<const uint32_t *>(sb);
+      const uint32_t body = (m.hoff + Hdr<kDelta, S>::bytes) * 8;
+      // |sum of differences| < 2^bits(len) * 2^(l-1)
+      if (S == 4 || (l ? l - 1 : 0u) + bits_of(len) <= 31) delta_block_staged<T, int32_t>(w32, body, l, x0, len, outp + base, wt);
+      else delta_block_staged<T, int64_t>(w32, body, l, x0, len, outp + base, wt);
+    }
+    if (!has_next) return;
+    ok = mbar_wait_bounded(&bar[cur ^ 1], ph[cur ^ 1]);
+    ph[cur ^ 1] ^= 1;
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) atomicOr(a.error, kErrTimeout);
+      return;
+    }
+    blk = nxt;
+  }
+}
+
 // ---- compressed-domain sum ----------------------------------------------------
 // Sum of decoded values mod 2^64 without writing them: reads only the payload.
 template <typename T, int CODEC>
@@ -359,11 +562,17 @@ static void run_decode(const DecodeLaunch &L, cudaStream_t st) {
     else decode_kernel<T, CODEC><<<(unsigned)nblk, 256, 0, st>>>(L);
     return;
   }
-  const int smem = 2 * kStageBuf + 64;  // +64: field reads may run a few bytes past a full buffer
-  const LaunchInfo i = launch_info<decode_staged_kernel<T, CODEC, false>>(256, smem);
-  if (i.error != cudaSuccess) return;  // the caller reports it
-  const uint64_t grid = umin64(nblk, (uint64_t)i.sms * (uint64_t)i.per_sm);
-  decode_staged_kernel<T, CODEC><<<(unsigned)grid, 256, smem, st>>>(L, kStageBuf);
+  // +128: field reads may run past a full buffer, a Delta span's by up to 68 bytes
+  const int smem = 2 * kStageBuf + 128;
+  if constexpr (CODEC == kDelta) {
+    const LaunchInfo i = launch_info<decode_delta_kernel<T>>(256, smem);
+    if (i.error != cudaSuccess) return;  // the caller reports it
+    decode_delta_kernel<T><<<(unsigned)umin64(nblk, (uint64_t)i.sms * (uint64_t)i.per_sm), 256, smem, st>>>(L, kStageBuf);
+  } else {
+    const LaunchInfo i = launch_info<decode_staged_kernel<T, CODEC, false>>(256, smem);
+    if (i.error != cudaSuccess) return;  // the caller reports it
+    decode_staged_kernel<T, CODEC><<<(unsigned)umin64(nblk, (uint64_t)i.sms * (uint64_t)i.per_sm), 256, smem, st>>>(L, kStageBuf);
+  }
 }
 int launch_decode(int codec, int s, const DecodeLaunch &L, cudaStream_t st) { LECO_DISPATCH(codec, s, run_decode, L, st); }
 
