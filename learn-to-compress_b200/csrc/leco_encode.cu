@@ -49,10 +49,8 @@ __global__ void __launch_bounds__(256) encode_legacy_kernel_warp(EncodeArgs a, u
 // then adds the 32 values of block j to its running sums in order, exactly the
 // reference's loop (lr.h:72-77; Y sums of polynomial_regression_internals.hpp:129-137).
 // A full tile's 32 conversions and products are taken before its adds, so the
-// lane's critical path is the add chains alone (the loop that waited on a load and
-// a conversion at every step took ~200 us per block of 4096 values).  Twelve warps
-// per SM (registers) hold a whole 200M-value column's 1526 warps in one wave, where
-// the loads are in flight across warps; a lone warp waits for each next tile.
+// lane's critical path is the add chains alone.  For values that the ring kernel
+// below cannot copy in 16-byte pieces.
 template <typename T, int CODEC>
 __global__ void __launch_bounds__(128) seq_fit_tiled_kernel(const T *__restrict__ values, uint64_t n, uint32_t bs,
                                                             uint64_t nb, PolyX px, double *__restrict__ models) {
@@ -119,17 +117,17 @@ __global__ void __launch_bounds__(128) seq_fit_tiled_kernel(const T *__restrict_
   if (len) store_seq_model<CODEC>(models + mine * 3, s0, s1, s2, len, bs, px.x);
 }
 
-// The same fits with a deeper pipeline per warp, for columns whose warps fit in one
-// wave of this kernel (four CTAs per SM): one warp per CTA, lane j fits block b0 + j,
+// The same fits with a deeper pipeline per warp: one warp per CTA, lane j fits block b0 + j,
 // and a ring of kFitStages stages holds the next tiles of all 32 blocks (row j: block
 // b0 + j, padded by 16 bytes so that the lanes' 16-byte reads of their own rows spread
 // over the banks).  A stage is filled by coalesced 16-byte cp.async copies (one group
-// per stage) and read after the warp has waited for its group, so a lone warp's add
-// chains are no longer held up by its loads (one block of 4096 values: ~60 us instead
-// of ~110 us).  Needs 16-byte aligned values and bs * sizeof(T) a multiple of 16.
+// per stage) and read after the warp has waited for its group.  Four stages leave six
+// warps per SM (888: a 28,000-block column in one wave): encode of 100M u64 values 482 us
+// with three, 491 with four, 507 with six; of 200M 936, 910, 913; 522 (100M) with the tiled
+// kernel above.  Needs 16-byte aligned values and bs * sizeof(T) a multiple of 16.
 // Tiles of fewer than 32 values (a block's last when bs is not a multiple of 32, the
 // column's short last block) are read from global memory directly.
-constexpr int kFitStages = 6;
+constexpr int kFitStages = 4;
 template <typename T>
 __host__ __device__ constexpr uint32_t fit_row_bytes() { return 32u * sizeof(T) + 16u; }
 template <typename T>
@@ -223,12 +221,18 @@ __global__ void __launch_bounds__(32) seq_fit_ring_kernel(const T *__restrict__ 
 
 // ---- host launchers ---------------------------------------------------------------
 
-// u64 LeCo columns of at least this many blocks take the fits from the kernels below, which
-// read the values once more but run at memory speed (100M values, 24,415 blocks: 190 us), and
-// leave the row encoder without its own (100M: 603 us with the fits inside, 522 us with the
-// fit pass).  A short column's fit kernel is bound by one block's chains of dependent additions
-// (71 us for 4096 values, one block or thousands), which the row encoder does not have.
-constexpr uint64_t kSeqFitBlocks = 16384;
+// Columns of at least this many blocks take the fits from the kernels below, which read the
+// values once more but at up to 6 TB/s, and leave the row encoder without its own.  A short
+// column's fit kernel is bound by one block's chain of dependent additions (71 us for 4096
+// values, one block or thousands), which the row encoder does not have.  u64, us with the fit
+// kernel / with the fits inside:
+//   blocks of 4096 values, LeCo:   4096: 147 / 114   8192: 200 / 207   12288: 257 / 298   24576: 485 / 599
+//   blocks of 1000 values, LeCo:   4096:  52 /  42   8192:  73 /  69   12288:  99 / 112   24576: 168 / 199
+//   blocks of 4096 values, poly2:  4096: 154 / 143   8192: 218 / 284   12288: 278 / 431   24576: 537 / 883
+//   blocks of 1000 values, poly2:  4096:  53 /  51   8192:  73 /  91   12288:  98 / 143   24576: 183 / 279
+// u32 LeCo columns keep the fits inside at every size: their sums seldom reach 2^53, so the
+// row encoder takes them from its scan.
+constexpr uint64_t kSeqFitBlocks = 8192, kSeqFitBlocksPoly = 5120;
 // The sequential fits of a column's blocks into L.seq_models (CODEC: kLinear, also for the
 // legacy codec, or kPoly2).
 template <typename T, int CODEC>
@@ -237,11 +241,8 @@ static int launch_seq_fit(const EncodeLaunch &L, cudaStream_t st) {
   for (int i = 0; i < 10; ++i) px.x[i] = L.polyX[i];
   // four warps per CTA, 32 blocks per warp
   const uint64_t warps = (L.nb + 31) / 32;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const T *values = reinterpret_cast<const T *>(L.values);
-  if (warps <= 4ull * (uint64_t)sms && (reinterpret_cast<uintptr_t>(L.values) & 15) == 0 && ((uint64_t)L.bs * sizeof(T)) % 16 == 0) {
+  if ((reinterpret_cast<uintptr_t>(L.values) & 15) == 0 && ((uint64_t)L.bs * sizeof(T)) % 16 == 0) {
     constexpr uint32_t fsm = fit_smem_bytes<T>();
     if (fsm > 48 * 1024) cudaFuncSetAttribute(seq_fit_ring_kernel<T, CODEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm);
     seq_fit_ring_kernel<T, CODEC><<<(unsigned)warps, 32, fsm, st>>>(values, L.n, L.bs, L.nb, px, L.seq_models);
@@ -259,8 +260,10 @@ int launch_encode(int codec, int s, const EncodeLaunch &L, cudaStream_t st) {
   for (int i = 0; i < 10; ++i) a.polyX[i] = L.polyX[i];
   if (codec != kLegacy) {
     const bool ref = L.seq_models != nullptr;
-    if (ref && codec == kLinear && s == 8 && L.nb >= kSeqFitBlocks) {
-      launch_seq_fit<uint64_t, kLinear>(L, st);
+    if (ref && (codec == kLinear ? s == 8 && L.nb >= kSeqFitBlocks : L.nb >= kSeqFitBlocksPoly)) {  // (FOR and Delta: never ref)
+      if (codec == kLinear) launch_seq_fit<uint64_t, kLinear>(L, st);
+      else if (s == 8) launch_seq_fit<uint64_t, kPoly2>(L, st);
+      else launch_seq_fit<uint32_t, kPoly2>(L, st);
       a.seq_models = L.seq_models;
     }
     return s == 4 ? launch_rows_u32(codec, a, ref, st) : launch_rows_u64(codec, a, ref, st);

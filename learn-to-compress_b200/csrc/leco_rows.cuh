@@ -34,7 +34,8 @@
 // rest barriers within the block and the wait for the item's offset).  Against the encoder
 // with one CTA per block that gathered each output chunk field by field, or staged twice:
 // one 4096-value u64 block 82 -> 18 us, 1M u32 LeCo in blocks of 1000 34.8 -> 19 us, 30M u32
-// FOR 130 -> 62 us, 20M u64 Delta in blocks of 2048 176 -> 77 us, 100M u64 LeCo 557 -> 522 us.
+// FOR 130 -> 62 us, 20M u64 Delta in blocks of 2048 176 -> 77 us, 100M u64 LeCo (fits from the
+// fit kernel, leco_encode.cu) 557 -> 491 us.
 #pragma once
 #include "leco_encode.cuh"
 

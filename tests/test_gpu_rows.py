@@ -50,9 +50,9 @@ def test_images_match_oracle(lc, orc, dev, s, bs):
     lc.check()
 
 
-@pytest.mark.parametrize("n", [4096 * 16383, 4096 * 16384 + 5])
+@pytest.mark.parametrize("n", [4096 * 8191, 4096 * 8192 + 5])
 def test_large_column_fit_paths_agree(lc, dev, n):
-    """The fit inside the row encoder (fewer than 16384 blocks) and the fit kernels (from
+    """The fit inside the row encoder (fewer than 8192 blocks) and the fit kernels (from
     there on) leave the same images: the first blocks of a column are those of a short one."""
     import torch
 
