@@ -33,9 +33,9 @@
 // u64 Delta 6.2K, u64 LeCo 8.8K, with the fit's chains 12.6K; issue slots 45-60 % busy, the
 // rest barriers within the block and the wait for the item's offset).  Against the encoder
 // with one CTA per block that gathered each output chunk field by field, or staged twice:
-// one 4096-value u64 block 82 -> 18 us, 1M u32 LeCo in blocks of 1000 34.8 -> 19 us, 30M u32
-// FOR 130 -> 62 us, 20M u64 Delta in blocks of 2048 176 -> 77 us, 100M u64 LeCo (fits from the
-// fit kernel, leco_encode.cu) 557 -> 491 us.
+// one 4096-value u64 block 82 -> 13 us (host-bound), 1M u32 LeCo in blocks of 1000 34.8 -> 16 us,
+// 30M u32 FOR 130 -> 55 us, 20M u64 Delta in blocks of 2048 176 -> 68 us, 100M u64 LeCo (fits
+// from the fit kernel, leco_encode.cu) 557 -> 450 us.
 #pragma once
 #include "leco_encode.cuh"
 
@@ -55,7 +55,7 @@ __host__ __device__ constexpr int rows_sums(int codec) { return codec == kLinear
 
 // Shared memory of one CTA of nt threads in groups of R.
 struct RowsLayout {
-  uint32_t tab, base, mask, wtot, red, hdr, model, size, goff, total;
+  uint32_t tab, base, mask, wtot, red, hdr, model, size, goff, count, total;
 };
 __host__ __device__ constexpr RowsLayout rows_layout(uint32_t nt, uint32_t R, uint32_t s, uint32_t ns) {
   RowsLayout L{};
@@ -70,6 +70,7 @@ __host__ __device__ constexpr RowsLayout rows_layout(uint32_t nt, uint32_t R, ui
   L.model = o; o += ng * 32;                // double [groups][4]
   L.size = o;  o += ng * 8;                 // u64 [groups]
   L.goff = o;  o += ng * 8;                 // u64 [groups]
+  L.count = o; o += 8;                      // u32: groups whose size is known
   L.total = o;
   return L;
 }
@@ -885,6 +886,8 @@ struct RowCoded {
 template <typename T, int CODEC, bool FULL, uint32_t RT>
 __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const RowPass<T, RT> &P, bool ref, uint32_t sb, uint8_t *smem,
                                                    const RowsLayout &L, uint64_t b, RowCoded &C, uint64_t *status) {
+  uint64_t *sizes = reinterpret_cast<uint64_t *>(smem + L.size);
+  uint32_t *count = reinterpret_cast<uint32_t *>(smem + L.count);
   constexpr uint32_t S = sizeof(T), TB = 8 * S, V = 16 / S;
   const RowGroup<RT> &g = P.g;
   const uint32_t len = P.len, cnt = P.cnt, p0 = 32 * g.rank;
@@ -905,8 +908,20 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
     // FOR_integer_template.h:89, poly_fix_integer_template.h:121), so a packed block of
     // that width would not decode there.  Delta has no such rule.
     if (CODEC != kDelta && l == TB - 1) l = TB;
-    // an item of one block publishes its size here, before its fields are made
-    if (status && g.rank == 0) st_relaxed(status, kFlagAgg | image_size<CODEC, S>(l, len));
+    // The item's total goes out when its last block has its width, before the fields are made.
+    if (g.rank == 0) {
+      const uint32_t NB = g.nt / g.R();
+      sizes[g.gi] = image_size<CODEC, S>(l, len);
+      if (status) {
+        __threadfence_block();
+        if (NB == 1 || atomicAdd(count, 1u) == NB - 1) {
+          __threadfence_block();
+          uint64_t total = 0;
+          for (uint32_t k = 0; k < NB; ++k) total += reinterpret_cast<volatile uint64_t *>(sizes)[k];
+          st_relaxed(status, kFlagAgg | total);
+        }
+      }
+    }
     return l;
   };
   if constexpr (CODEC == kLinear || CODEC == kPoly2) {
@@ -1166,14 +1181,17 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
 
 // ---- offsets of a column's items ------------------------------------------------------
 // A single column's items take their byte offsets from a publisher CTA: it walks the status
-// words in item order, kPubWords per thread and step, and turns every published total into an
+// words in item order, kPubWindow of them a step, and turns every published total into an
 // inclusive prefix once all the items before it have published theirs.  An item publishes
 // its total, packs, and then polls its own word alone. Waits are bounded: on expiry the error word
 // is set and the item is not written.
-constexpr uint32_t kPubWords = 8;
+// The items in flight (~900 to 1500) wait for the step, and a step is a read of L2 and two
+// barriers, so its width matters both ways: 24.6M u32 FOR / Delta values, us: windows of 128
+// words 47 / 48, 256 42 / 44, 512 41 / 44, 1024 50 / 51; one warp stepping over 256 words 47 / 50.
+constexpr uint32_t kPubWindow = 512;
 template <uint32_t NT>
 __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, uint32_t *error, uint8_t *smem) {
-  constexpr uint32_t NW = NT / 32;
+  constexpr uint32_t NW = NT / 32, kPubWords = kPubWindow / NT;
   uint64_t *wsum = reinterpret_cast<uint64_t *>(smem);                // [2][NW]
   uint32_t *wfirst = reinterpret_cast<uint32_t *>(smem + 2 * NW * 8);  // [2][NW]
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -1280,11 +1298,12 @@ __device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t i
   uint64_t *hdr = reinterpret_cast<uint64_t *>(smem + L.hdr) + 4 * g.gi;
   uint64_t *sizes = reinterpret_cast<uint64_t *>(smem + L.size), *goffs = reinterpret_cast<uint64_t *>(smem + L.goff);
 
+  if (g.row == 0) *reinterpret_cast<uint32_t *>(smem + L.count) = 0;
   stage_rows<T>(g, sb, reinterpret_cast<const T *>(a.values) + b * a.bs, len);
-  g.sync();
+  __syncthreads();
   RowCoded C{};
   // (the two ways meet at the same barriers: the warps of a block may differ)
-  uint64_t *status = PUB && !alone && NB == 1 ? a.status + item : nullptr;
+  uint64_t *status = alone ? nullptr : a.status + item;
   if (__all_sync(0xffffffffu, P.cnt == 32)) encode_rows_passes<T, CODEC, true>(a, P, ref, sb, smem, L, b, C, status);
   else encode_rows_passes<T, CODEC, false>(a, P, ref, sb, smem, L, b, C, status);
   const uint32_t l = C.l;
@@ -1292,7 +1311,6 @@ __device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t i
   const uint32_t H = raw ? 1u : Hdr<CODEC, S>::bytes;
   const uint64_t size = image_size<CODEC, S>(l, len);
   if (g.rank == 0) {
-    sizes[g.gi] = size;
     uint64_t v0 = 0, v1 = 0, v2 = 0;
     if (!raw) {
       if (CODEC == kLinear || CODEC == kPoly2) {
@@ -1320,7 +1338,6 @@ __device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t i
       if (g.lane >= d) incl += o;
     }
     total = __shfl_sync(0xffffffffu, (unsigned long long)incl, 31);
-    if (!status && (PUB || item) && g.lane == 0) st_relaxed(&a.status[item], kFlagAgg | total);
   }
   // ---- pack this row ----
   const uint32_t gb = sb + g.gi * R * (32 * S);
