@@ -67,7 +67,7 @@ __host__ __device__ constexpr RowsLayout rows_layout(uint32_t nt, uint32_t R, ui
   L.wtot = o;  o += 3 * nw * 8;             // double [3][warps]
   L.red = o;   o += 2 * 2 * nw * 8;         // u64 [2][2][warps]
   L.hdr = o;   o += ng * 32;                // u64 [groups][4]: header bytes
-  L.model = o; o += ng * 32;                // double [groups][4]
+  L.model = L.hdr;                          // double [groups][4]: read before the header is made
   L.size = o;  o += ng * 8;                 // u64 [groups]
   L.goff = o;  o += ng * 8;                 // u64 [groups]
   L.count = o; o += 8;                      // u32: groups whose size is known
