@@ -405,8 +405,8 @@ __device__ __forceinline__ uint32_t legacy_residuals(const EncSmem<T> &sm, doubl
 // One lane per block adds the block's values in the reference's own order and FP64
 // operations, so the model is bit-identical to lr_int_T::caltheta (lr.h:66-85) or to
 // the Y sums of polynomial_regression_iter (polynomial_regression_internals.hpp:129-137)
-// (the kernels: seq_fit_tiled_kernel and seq_fit_ring_kernel in leco_encode.cu,
-// batch_seq_fit_kernel in leco_batch.cu).
+// (the kernels: seq_fit_tiled_kernel and seq_fit_ring_kernel in leco_encode.cu; the row
+// encoder computes the same sums in parallel, leco_rows.cuh).
 struct PolyX {
   double x[10];
 };

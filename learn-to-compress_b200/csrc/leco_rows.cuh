@@ -6,8 +6,8 @@
 // between threads, residuals replace the values they came from, and nothing but running
 // maxima and sums stays in registers, so that six CTAs of four warps fit an SM.  A CTA of NT threads encodes NT / R consecutive blocks (an item) and
 // takes one look-back for all of them.  Used by the single-column kernels
-// (leco_encode.cu) and the batch engine (leco_batch_encode.cu); blocks keep the images of
-// encode_block byte for byte.
+// (leco_encode.cu) and the batch engine (leco_batch_encode.cu); blocks are the
+// reference's images byte for byte.
 //
 // The reference's fit adds a block's values (and i * value, i * i * value) one after the
 // other in FP64 (lr.h:72-77, polynomial_regression_internals.hpp:129-137).  rows_fit
