@@ -52,6 +52,15 @@ namespace {
 // Shared memory one work item may take (the CTA limit is 227 KB).
 constexpr uint32_t kBatchMaxSmem = 200 * 1024;
 
+// The most shared memory an encoder item can take (any codec, value type and block size).  A
+// kernel's opt-in to more than 48 KB belongs to the kernel, not to the batch: set to one batch's
+// own size it would take a smaller batch's after that one was made.
+int batch_enc_max_smem(int which) {
+  uint32_t m = 0;
+  for (uint32_t R = which ? 512 : 8; R <= (which ? 512u : 256u); R <<= 1) m = std::max(m, rows_layout(which ? 512 : 256, R, 8, 3).total);
+  return (int)m;
+}
+
 int berr(int code, const std::string &m) { return leco::record_error(code, m); }
 
 bool needs_seq(int codec, int dtype, uint32_t bs, int fit_mode) {
@@ -183,10 +192,10 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
     e = cudaMemcpy(b->d_enc_items, enc_items.data(), enc_items.size() * sizeof(uint64_t), cudaMemcpyHostToDevice);
   if (e == cudaSuccess && leco::device_error_word(&b->err)) e = cudaErrorUnknown;
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess && b->enc_smem[0] > 48 * 1024)
-    e = cudaFuncSetAttribute(batch_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->enc_smem[0]);
-  if (e == cudaSuccess && b->enc_smem[1] > 48 * 1024)
-    e = cudaFuncSetAttribute(batch_encode_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->enc_smem[1]);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(batch_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_enc_max_smem(0));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(batch_encode_large_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, batch_enc_max_smem(1));
   int sms = 148, per_enc[2] = {1, 1}, per_dec = 1;
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
   if (e == cudaSuccess && b->enc_n[0])
