@@ -279,7 +279,8 @@ int launch_encode(int codec, int s, const EncodeLaunch &L, cudaStream_t st) {
     encode_legacy_kernel_warp<<<(unsigned)((L.nb + 7) / 8), 256, 8 * slice, st>>>(a, slice);
     return 0;
   }
-  if (smem > 48 * 1024) cudaFuncSetAttribute(encode_legacy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (smem > 48 * 1024)  // the largest block's limit: the kernel's, not this call's
+    cudaFuncSetAttribute(encode_legacy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)enc_smem_bytes(LECO_MAX_BLOCK, 4));
   encode_legacy_kernel<<<(unsigned)L.nb, 256, smem, st>>>(a);
   return 0;
 }

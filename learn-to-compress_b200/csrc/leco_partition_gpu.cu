@@ -895,8 +895,8 @@ int leco_varlen_partition_device(const uint64_t *d_values, uint64_t n, uint32_t 
   if (bs <= kPartCtaMax) {
     const uint32_t smem = part_smem_bytes(bs);
     cudaError_t se = cudaSuccess;
-    if (smem > 48 * 1024)
-      se = cudaFuncSetAttribute(partition_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024)  // the largest block's limit: it is the kernel's, and another thread may be about to launch one
+      se = cudaFuncSetAttribute(partition_cta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)part_smem_bytes(kPartCtaMax));
     int dev = 0, sms = 148, per_sm = 1;
     if (se == cudaSuccess) se = cudaGetDevice(&dev);
     if (se == cudaSuccess) se = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

@@ -542,9 +542,10 @@ int leco_varlen_encode(const uint64_t *d_values, uint64_t n, const uint64_t *d_s
             reinterpret_cast<uint32_t *>(ws + status_bytes), err, exact, max_segment_len, exact ? nullptr : models};
   cudaError_t e = cudaMemsetAsync(ws, 0, status_bytes + 256, st);
   if (e == cudaSuccess && !exact) varlen_seq_fit_kernel<<<(unsigned)((nseg + 127) / 128), 128, 0, st>>>(d_values, n, d_starts, nseg, models);
-  const int smem = 8 * max_segment_len + (max_segment_len / 32 + 9) * 4;
-  if (e == cudaSuccess && smem > 48 * 1024)
-    e = cudaFuncSetAttribute(varlen_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  auto smem_bytes = [](uint32_t len) { return (int)(8 * len + (len / 32 + 9) * 4); };
+  const int smem = smem_bytes(max_segment_len);
+  if (e == cudaSuccess && smem > 48 * 1024)  // the largest segment's limit: the kernel's, not this call's
+    e = cudaFuncSetAttribute(varlen_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(kVarlenMaxSeg));
   if (e == cudaSuccess) varlen_encode_kernel<<<(unsigned)nseg, 128, smem, st>>>(a);  // 128 threads: more segments in flight per SM
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? LECO_OK : verr(LECO_ERR_CUDA, std::string("leco_varlen_encode: ") + cudaGetErrorString(e));

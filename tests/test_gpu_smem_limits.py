@@ -28,3 +28,43 @@ def test_older_batch_encodes_after_a_smaller_one(lc, dev, big, small):
             assert torch.equal(c.offsets, one.offsets)
             assert torch.equal(c.payload[: one.nbytes], one.payload[: one.nbytes])
     lc.check()
+
+
+@pytest.mark.parametrize("op", ["partition", "varlen", "legacy"])
+def test_threads_with_different_block_sizes(lc, dev, op):
+    """Two host threads, one with blocks that need the opt-in in full and one with smaller ones:
+    every call of both succeeds."""
+    import threading
+
+    import torch
+
+    rng = np.random.default_rng(7)
+    x = np.cumsum(rng.integers(0, 5000, 64_000, dtype=np.uint64)) + np.uint64(1 << 40)
+    xd, xs = to_dev(x, dev), to_dev((x & np.uint64(0xFFFFFFF)).astype(np.uint32), dev)
+    sizes = {"partition": (8000, 4000), "varlen": (16_000, 6_400), "legacy": (16_000, 12_800)}[op]
+    errors = []
+
+    def work(bs):
+        s = torch.cuda.Stream()
+        try:
+            with torch.cuda.stream(s):
+                if op == "varlen":
+                    starts = torch.arange(0, len(x), bs, device=dev, dtype=torch.int64)
+                for _ in range(300):
+                    if op == "partition":
+                        lc.varlen_partition_device(xd[: 2 * bs], 2, 12)
+                    elif op == "varlen":
+                        lc.varlen_encode(xd, starts, max_segment_len=bs)
+                    else:
+                        lc.encode(xs, 5, bs)
+            s.synchronize()
+        except Exception as e:  # noqa: BLE001 (reported below)
+            errors.append((bs, e))
+
+    threads = [threading.Thread(target=work, args=(bs,)) for bs in sizes]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    lc.check()
