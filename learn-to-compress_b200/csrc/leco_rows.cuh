@@ -1180,10 +1180,11 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
 }
 
 // ---- offsets of a column's items ------------------------------------------------------
-// A single column's items take their byte offsets from a publisher CTA: it walks the status
+// A single column's items take their byte offsets from a publisher CTA, the first CTA of the
+// column to start (items are numbered in the order in which theirs started): it walks the status
 // words in item order, kPubWindow of them a step, and turns every published total into an
 // inclusive prefix once all the items before it have published theirs.  An item publishes
-// its total, packs, and then polls its own word alone. Waits are bounded: on expiry the error word
+// its total, packs, and then polls its own word alone.  Waits are bounded: on expiry the error word
 // is set and the item is not written.
 // The items in flight (~900 to 1500) wait for the step, and a step is a read of L2 and two
 // barriers, so its width matters both ways: 24.6M u32 FOR / Delta values, us: windows of 128

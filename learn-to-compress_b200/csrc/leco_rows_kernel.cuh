@@ -15,15 +15,26 @@ constexpr int rows_min_ctas() {
 }
 
 // One CTA of NT threads per item of NT / R blocks (RT: R when it is 64 or more, else 0).  A
-// column of one item needs no other; else CTA 0 is the publisher and CTA i + 1 takes item i:
-// CTAs start in the order of their index, so the publisher runs before any item and every
-// item it waits for has started.
+// column of one item needs no other; else the CTAs take their roles from a ticket as they
+// start, since CUDA does not promise the order of their indexes: the first is the publisher,
+// the k-th after it takes item k - 1, so whatever an item waits for has started before it.
+// The ticket is a trip to L2 before the first load (roles by index / by ticket: 100M u64 LeCo
+// 455 / 464 us, 30M u32 FOR 56.7 / 59.4, 20M u64 Delta 67.6 / 71.0; CTAs that stay and ask for
+// their next ticket ahead: 574, 71, 76).
 template <typename T, int CODEC, int NT, uint32_t RT>
 __global__ void __launch_bounds__(NT, rows_min_ctas<T, CODEC, NT>()) encode_rows_kernel(EncodeArgs a, uint32_t R, uint32_t items,
                                                                                          bool ref) {
   extern __shared__ __align__(256) uint8_t smem_raw[];
-  if (items > 1 && blockIdx.x == 0) publish_items<NT>(a.status, items, a.error, smem_raw);
-  else encode_rows_item<T, CODEC, RT, true>(a, items > 1 ? blockIdx.x - 1 : 0, R, ref, items == 1, smem_raw);
+  uint32_t role = 1;
+  if (items > 1) {
+    // (the place of the groups' offsets, which are written after further barriers)
+    uint32_t *ticket = reinterpret_cast<uint32_t *>(smem_raw + rows_layout(NT, RT ? RT : R, sizeof(T), rows_sums(CODEC)).goff);
+    if (threadIdx.x == 0) *ticket = atomicAdd(a.ticket, 1u);
+    __syncthreads();
+    role = *ticket;
+  }
+  if (role == 0) publish_items<NT>(a.status, items, a.error, smem_raw);
+  else encode_rows_item<T, CODEC, RT, true>(a, role - 1, R, ref, items == 1, smem_raw);
 }
 
 template <typename T, int CODEC, int NT, uint32_t RT>
