@@ -470,6 +470,11 @@ int leco_check(leco_stream_t stream);
  * returns what leco_check reports afterwards: LECO_ERR_TIMEOUT when the bounded
  * wait gave up as designed (*h_result = ~0).  Synchronous; the context stays usable. */
 int leco_test_bounded_wait(uint32_t spin_limit, uint64_t *h_result);
+/* TEST HOOK of the same kind for the column encoder's waits: part 0 runs its publisher on
+ * three items of which only the first has published its total (48), part 1 an item's wait
+ * for a publisher that never comes.  h_words (4 words): the items' three status words and,
+ * for part 1, the wait's result (~0 when it gave up). */
+int leco_test_rows_wait(uint32_t spin_limit, int part, uint64_t *h_words);
 /* Message of the last error on this thread ("" if none). */
 const char *leco_last_error(void);
 /* Library version string. */

@@ -8,7 +8,7 @@
 // Delta_int<T>::encodeArray8_int (delta_integer_template.h:26-87),
 // Leco_int_poly<T,2>::encodeArray8_int (poly_fix_integer_template.h:28-91),
 // packers write_delta_int_T / write_FOR_int_T (bit_write.h:257-390).
-#include "leco_encode.cuh"
+#include "leco_rows.cuh"
 
 #include <string>
 
@@ -285,32 +285,67 @@ int launch_encode(int codec, int s, const EncodeLaunch &L, cudaStream_t st) {
   return 0;
 }
 
-// Bounded-wait check: block 1 of a two-block look-back whose block 0 never
-// publishes its size (a status word nothing sets).  The wait must give up after
-// `spin_limit` polls, set the error word and return.
+// Bounded-wait checks.  Block 1 of a two-block look-back whose block 0 never publishes its
+// size (a status word nothing sets): the wait must give up after `spin_limit` polls, set the
+// error word and return.
 __global__ void lookback_timeout_probe_kernel(uint64_t *status, uint32_t *error, uint32_t spin_limit, uint64_t *result) {
   if (threadIdx.x < 32) {
     const uint64_t excl = lookback_prefix(status, 1, 16, error, spin_limit);
     if (threadIdx.x == 0) *result = excl;
   }
 }
+// The row encoder's two waits: the publisher of three items of which the second never
+// publishes its total (part 0), and an item whose word the publisher never reaches (part 1).
+__global__ void __launch_bounds__(128) rows_timeout_probe_kernel(uint64_t *status, uint32_t *error, uint32_t spin_limit, int part,
+                                                                 uint64_t *result) {
+  __shared__ __align__(16) uint8_t scratch[256];
+  if (part == 0) {
+    if (threadIdx.x == 0) status[0] = kFlagAgg | 48;
+    __syncthreads();
+    publish_items<128>(status, 3, error, scratch, spin_limit);
+  } else if (threadIdx.x == 0) {
+    *result = await_prefix(status, 1, 16, error, spin_limit);
+  }
+}
 
 }  // namespace leco
 
-extern "C" int leco_test_bounded_wait(uint32_t spin_limit, uint64_t *h_result) {
+// Runs `launch(words, error word)` on four zeroed words and reports what leco_check says;
+// h_words: the words afterwards.
+template <typename Launch>
+static int run_wait_probe(const char *what, uint64_t (&h_words)[4], Launch launch) {
   using namespace leco;
   uint32_t *err = nullptr;
   int rc = device_error_word(&err);
   if (rc) return rc;
-  uint64_t *buf = nullptr;  // [2] status words + [1] result
-  cudaError_t e = cudaMalloc(&buf, 3 * sizeof(uint64_t));
-  if (e == cudaSuccess) e = cudaMemset(buf, 0, 3 * sizeof(uint64_t));
+  uint64_t *buf = nullptr;
+  cudaError_t e = cudaMalloc(&buf, sizeof h_words);
+  if (e == cudaSuccess) e = cudaMemset(buf, 0, sizeof h_words);
   if (e == cudaSuccess) {
-    lookback_timeout_probe_kernel<<<1, 32>>>(buf, err, spin_limit, buf + 2);
+    launch(buf, err);
     e = cudaDeviceSynchronize();
   }
-  if (e == cudaSuccess && h_result) e = cudaMemcpy(h_result, buf + 2, sizeof(uint64_t), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(h_words, buf, sizeof h_words, cudaMemcpyDeviceToHost);
   if (buf) cudaFree(buf);
-  if (e != cudaSuccess) return record_error(LECO_ERR_CUDA, std::string("leco_test_bounded_wait: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) return record_error(LECO_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
   return leco_check(nullptr);
+}
+
+extern "C" int leco_test_bounded_wait(uint32_t spin_limit, uint64_t *h_result) {
+  uint64_t words[4] = {0, 0, 0, 0};
+  const int rc = run_wait_probe("leco_test_bounded_wait", words, [&](uint64_t *w, uint32_t *err) {
+    leco::lookback_timeout_probe_kernel<<<1, 32>>>(w, err, spin_limit, w + 3);
+  });
+  if (h_result) *h_result = words[3];
+  return rc;
+}
+
+extern "C" int leco_test_rows_wait(uint32_t spin_limit, int part, uint64_t *h_words) {
+  if (part < 0 || part > 1 || !h_words) return leco::record_error(LECO_ERR_ARG, "leco_test_rows_wait: part 0 or 1, four words");
+  uint64_t words[4] = {0, 0, 0, 0};
+  const int rc = run_wait_probe("leco_test_rows_wait", words, [&](uint64_t *w, uint32_t *err) {
+    leco::rows_timeout_probe_kernel<<<1, 128>>>(w, err, spin_limit, part, w + 3);
+  });
+  for (int i = 0; i < 4; ++i) h_words[i] = words[i];
+  return rc;
 }

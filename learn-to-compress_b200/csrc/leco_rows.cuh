@@ -1191,7 +1191,8 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
 // words 47 / 48, 256 42 / 44, 512 41 / 44, 1024 50 / 51; one warp stepping over 256 words 47 / 50.
 constexpr uint32_t kPubWindow = 512;
 template <uint32_t NT>
-__device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, uint32_t *error, uint8_t *smem) {
+__device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, uint32_t *error, uint8_t *smem,
+                                              uint32_t spin_limit = kSpinLimit) {
   constexpr uint32_t NW = NT / 32, kPubWords = kPubWindow / NT;
   uint64_t *wsum = reinterpret_cast<uint64_t *>(smem);                // [2][NW]
   uint32_t *wfirst = reinterpret_cast<uint32_t *>(smem + 2 * NW * 8);  // [2][NW]
@@ -1248,7 +1249,7 @@ __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, 
     uint64_t *carry = reinterpret_cast<uint64_t *>(smem + 2 * NW * 12);
     if (has_last) carry[par] = last;
     if (n == 0) {
-      if (++spins > kSpinLimit) {
+      if (++spins > spin_limit) {
         if (t == 0) atomicOr(error, kErrTimeout);
         return;
       }
@@ -1264,12 +1265,13 @@ __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, 
 }
 // One warp: the item's exclusive prefix, once the publisher has replaced its total by the
 // inclusive prefix; ~0 when the wait gave up.
-__device__ __forceinline__ uint64_t await_prefix(const uint64_t *status, uint64_t item, uint64_t total, uint32_t *error) {
+__device__ __forceinline__ uint64_t await_prefix(const uint64_t *status, uint64_t item, uint64_t total, uint32_t *error,
+                                                 uint32_t spin_limit = kSpinLimit) {
   uint32_t spins = 0;
   for (;;) {
     const uint64_t v = ld_relaxed(&status[item]);
     if ((v >> 62) == 2) return (v & kValMask) - total;
-    if (++spins > kSpinLimit) {
+    if (++spins > spin_limit) {
       atomicOr(error, kErrTimeout);
       return ~0ull;
     }

@@ -26,3 +26,20 @@ def test_every_role_is_a_ticket(lc, dev, s, codec, n, bs, items):
     assert np.array_equal(words[:items], np.uint64(2 << 62) | off[np.minimum(np.arange(1, items + 1) * per, nb)])
     assert torch.equal(col.decode(), x)
     lc.check()
+
+
+@pytest.mark.parametrize("part", [0, 1])
+def test_waits_run_out(lc, dev, part):
+    """The publisher waiting for an item's total and an item waiting for its prefix both give up
+    after their poll limit and report it; what had been published before stays, the rest is not
+    touched, and the context keeps working."""
+    import ctypes
+
+    words = (ctypes.c_uint64 * 4)()
+    assert lc.lib().leco_test_rows_wait(2000, part, words) == -5
+    lc.check()  # the error word was read and cleared
+    assert list(words) == ([(2 << 62) | 48, 0, 0, 0] if part == 0 else [0, 0, 0, 2**64 - 1])
+    x = to_dev(np.arange(50_000, dtype=np.uint64) * 3, dev)
+    col = lc.encode(x, lc.LINEAR, 1000)
+    assert col.decode().equal(x)
+    lc.check()
