@@ -308,6 +308,18 @@ __global__ void __launch_bounds__(kPartThreads) partition_kernel(PartitionArgs a
 // 2000, partition and encode: 43.7 ms with a thread per block, 4.47 ms with one warp per
 // block that scanned every class over all positions, 1.86 ms now.
 constexpr uint32_t kPartCtaMax = 8000;   // sizes fit 16 bits, shared memory fits an SM twice
+// A column of many short coarse blocks keeps the thread per block: a CTA's barriers and list
+// set-up take about 5 ns a block when all SMs are full, whatever its size, while a thread's
+// chain shortens with it.  CTA time over thread time, regime-switching column / random values:
+//   blocks:        4000         12000        25000        60000        300000
+//   of 4 values    1.1 / 1.2    1.7 / 1.8    2.5 / 2.7    3.5 / 3.8    4.9 / 5.3
+//   of 16          0.5 / 0.7    1.0 / 1.1    1.7 / 1.7    2.7 / 2.6    3.5 / 3.3
+//   of 32          0.4 / 0.4    0.7 / 0.6    1.1 / 0.9    1.7 / 1.4    2.1 / 1.7
+//   of 64          0.2 / 0.2    0.4 / 0.4    0.7 / 0.5    1.1 / 0.7    1.3 / 0.9
+//   of 80          0.2 / 0.2    0.4 / 0.3    0.6 / 0.4    1.0 / 0.6    1.2 / 0.8 (200000)
+//   of 96          0.2 / 0.1    0.3 / 0.2    0.5 / 0.3    0.8 / 0.5    0.9 / 0.6 (200000)
+constexpr uint32_t kPartThreadMax = 80;     // longest block of that kind
+constexpr uint32_t kPartThreadBlocks = 750;  // blocks per value of a block from which it is the faster
 constexpr uint32_t kPartLaneMax = 48;    // pairs of up to this many values: one lane each
 constexpr uint32_t kPartWarps = 4;
 constexpr uint32_t kPartPool = 192;      // merged segments whose extremes are in shared memory
@@ -892,7 +904,8 @@ int leco_varlen_partition_device(const uint64_t *d_values, uint64_t n, uint32_t 
   A.ticket = reinterpret_cast<uint32_t *>(w);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemsetAsync(A.ticket, 0, 4, st) != cudaSuccess) return record_error(LECO_ERR_CUDA, "leco_varlen_partition_device: memset");
-  if (bs <= kPartCtaMax) {
+  const bool many_short = bs <= kPartThreadMax && nb >= (uint64_t)kPartThreadBlocks * bs;
+  if (bs <= kPartCtaMax && !many_short) {
     const uint32_t smem = part_smem_bytes(bs);
     cudaError_t se = cudaSuccess;
     if (smem > 48 * 1024)  // the largest block's limit: it is the kernel's, and another thread may be about to launch one
