@@ -337,9 +337,12 @@ __device__ __forceinline__ void delta_block_staged(const uint32_t *words32, uint
 // CTA's threads leave an iteration together, with the next block's image landed: the barrier
 // that frees the buffer says so too, so a block of 4096 values has two barriers, not three.
 // 60M u64 values (0.58 GB, 91 us at the copy rate): 184 us with eight values per thread and
-// fields addressed one by one (67 instructions a value), 107 us now.
+// fields addressed one by one (67 instructions a value), 107 us now.  Raw u32 blocks are
+// written from the staged image, and u32 has five CTAs per SM: 60M random u32 values in blocks of
+// 513 / 1000 take 225 / 158 us (253 / 162 with four; read from global memory a second time,
+// 10M values in blocks of 1000 took 37 us instead of 29).
 template <typename T>
-__global__ void __launch_bounds__(256, 4) decode_delta_kernel(DecodeLaunch a, uint32_t bufcap) {
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 5 : 4) decode_delta_kernel(DecodeLaunch a, uint32_t bufcap) {
   constexpr int S = sizeof(T);
   extern __shared__ __align__(128) uint8_t stage[];
   __shared__ __align__(8) uint64_t bar[2];
@@ -390,8 +393,15 @@ __global__ void __launch_bounds__(256, 4) decode_delta_kernel(DecodeLaunch a, ui
     const uint32_t l = sb[m.hoff];
     const uint64_t base = blk * a.bs;
     const uint32_t len = (uint32_t)umin64(a.bs, a.n - base);
-    if (m.direct || l > 32 || l == 8u * S || len < 2) {
+    if (m.direct || l > 32 || len < 2) {
       decode_block<T, kDelta>(a, blk);
+    } else if (S == 4 && l == 32) {  // a raw u32 block: its words, out of the staged image
+      BlockHdr h;
+      h.l = l;
+      h.body_bit = (uint64_t)(m.hoff + 1) * 8;
+      const int32_t kstart = -(int32_t)((reinterpret_cast<uintptr_t>(outp + base) & 31) / S);  // groups start on 32 bytes
+      decode_narrow_mode<T, kDelta, kNarrowRaw, true, true, 256, false, 2>(h, reinterpret_cast<const uint32_t *>(sb), outp, base, 0,
+                                                                           len, kstart);
     } else {
       uint64_t x0 = 0;
 #pragma unroll
