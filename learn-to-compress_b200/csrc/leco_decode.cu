@@ -20,15 +20,19 @@
 
 namespace leco {
 
-// Direct decode: one CTA per block of the range, everything read from global memory.
+// Direct decode: one CTA per block of the range, everything read from global memory.  (Delta:
+// six CTAs of u32 per SM, and five of the warp kernel's for u64, as before the scan grew by its
+// 32-bit form: without that bound it takes 48 and 56 registers, and wide and raw blocks, which
+// do not use it, lose up to a fifth -- 60M random u64 in blocks of 32 703 -> 845 us, a range of
+// 20M random u32 in blocks of 513 95 -> 110 us.)
 template <typename T, int CODEC>
-__global__ void __launch_bounds__(256) decode_kernel(DecodeLaunch a) {
+__global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 4 ? 6 : 0) decode_kernel(DecodeLaunch a) {
   decode_block<T, CODEC>(a, a.first / a.bs + blockIdx.x);
 }
 
 // Small blocks: one warp per block, eight blocks per CTA.
 template <typename T, int CODEC>
-__global__ void __launch_bounds__(256) decode_kernel_warp(DecodeLaunch a, uint64_t nblk) {
+__global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 8 ? 5 : 0) decode_kernel_warp(DecodeLaunch a, uint64_t nblk) {
   const uint64_t i = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i < nblk) decode_block<T, CODEC, 32>(a, a.first / a.bs + i);
 }
