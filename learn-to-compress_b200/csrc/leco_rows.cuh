@@ -255,6 +255,26 @@ __device__ __forceinline__ void stage_rows(const RowGroup<RT> &g, uint32_t sb, c
   }
   cp_async_wait_all();
 }
+// Slot i of the row; with FULL false, values from cnt on read as 0.
+template <typename T, bool FULL>
+__device__ __forceinline__ void load_slot(uint32_t rowa, uint32_t cnt, uint32_t i, T *y) {
+  constexpr uint32_t V = 16 / sizeof(T);
+  const uint4 v = lds_v4(rowa ^ (i << 4));
+  if constexpr (sizeof(T) == 8) {
+    y[0] = ((uint64_t)v.y << 32) | v.x;
+    y[1] = ((uint64_t)v.w << 32) | v.z;
+  } else {
+    y[0] = v.x;
+    y[1] = v.y;
+    y[2] = v.z;
+    y[3] = v.w;
+  }
+  if (!FULL) {
+#pragma unroll
+    for (uint32_t k = 0; k < V; ++k)
+      if (V * i + k >= cnt) y[k] = 0;
+  }
+}
 // Calls slot(i, y) for the row's slots i = 0, 1, ... in order, y[] the slot's values; with
 // FULL false, values from cnt on read as 0.
 template <typename T, bool FULL, int UNROLL, typename Fn>
@@ -262,22 +282,8 @@ __device__ __forceinline__ void for_slots(uint32_t rowa, uint32_t cnt, Fn slot) 
   constexpr uint32_t V = 16 / sizeof(T), SL = 32 / V;
 #pragma unroll UNROLL
   for (uint32_t i = 0; i < SL; ++i) {
-    const uint4 v = lds_v4(rowa ^ (i << 4));
     T y[V];
-    if constexpr (sizeof(T) == 8) {
-      y[0] = ((uint64_t)v.y << 32) | v.x;
-      y[1] = ((uint64_t)v.w << 32) | v.z;
-    } else {
-      y[0] = v.x;
-      y[1] = v.y;
-      y[2] = v.z;
-      y[3] = v.w;
-    }
-    if (!FULL) {
-#pragma unroll
-      for (uint32_t k = 0; k < V; ++k)
-        if (V * i + k >= cnt) y[k] = 0;
-    }
+    load_slot<T, FULL>(rowa, cnt, i, y);
     slot(i, y);
   }
 }
@@ -754,23 +760,31 @@ __device__ __forceinline__ void lin_extremes(const RowPass<T, RT> &P, double m0,
   bad = 0;
   uint32_t high = 0;
   double ks = P.k0;
-  for_slots<T, FULL, 8 / V>(P.rowa, P.cnt, [&](uint32_t i, const T *y) {
-    int32_t d[V];
+  constexpr uint32_t SL = 32 / V, CH = 8 / V;  // slots of a row, slots of eight values
+#pragma unroll 1
+  for (uint32_t c = 0; c < SL; c += CH) {
 #pragma unroll
-    for (uint32_t j = 0; j < V; ++j) {
-      const double k = j ? __dadd_rn(ks, (double)j) : ks;
-      const double e = ceil_diff((uint64_t)y[j], __dadd_rn(m0, __dmul_rn(m1, k)));
-      d[j] = __double2loint(e);
-      const uint32_t fit = ((uint32_t)__double2hiint(e) + ((uint32_t)d[j] >> 31)) ^ 0x43380000u;
-      if (sizeof(T) == 8) high |= (uint32_t)((uint64_t)y[j] >> 32);
-      if (FULL || V * i + j < P.cnt) {
-        bad |= fit;
-        mx = max(mx, d[j]);
-        mn = min(mn, d[j]);
+    for (uint32_t q = 0; q < CH; ++q) {
+      T y[V];
+      load_slot<T, FULL>(P.rowa, P.cnt, c + q, y);
+#pragma unroll
+      for (uint32_t j = 0; j < V; ++j) {
+        const double k = j ? __dadd_rn(ks, (double)j) : ks;
+        const double e = ceil_diff((uint64_t)y[j], __dadd_rn(m0, __dmul_rn(m1, k)));
+        const int32_t d = __double2loint(e);
+        const uint32_t fit = ((uint32_t)__double2hiint(e) + ((uint32_t)d >> 31)) ^ 0x43380000u;
+        if (sizeof(T) == 8) high |= (uint32_t)((uint64_t)y[j] >> 32);
+        if (FULL || V * (c + q) + j < P.cnt) {
+          bad |= fit;
+          mx = max(mx, d);
+          mn = min(mn, d);
+        }
       }
+      ks = __dadd_rn(ks, (double)V);
     }
-    ks = __dadd_rn(ks, (double)V);
-  });
+    // a warp in which every row has failed leaves the block to the 64-bit pass
+    if (c == 0 && __all_sync(0xffffffffu, bad != 0 || high >> 19)) break;
+  }
   bad |= high >> 19;
   rg_reduce3<true>(P.g, mx, mn, bad, P.slots[0]);
 }
@@ -800,32 +814,41 @@ __device__ __forceinline__ uint32_t lin_residuals(const RowPass<T, RT> &P, doubl
 
 // The general residual passes: diff(y, j) gives a value's magnitude and sign (above: true)
 // at row position j.  wide_residuals puts signed 32-bit residuals over the values' place and
-// returns false when one does not fit (the values are gone then).  wide_extreme gives the
+// returns 0 when all fit, else kWide and, unless every warp saw that from its rows' first values
+// and left them alone, kGone: the values have been written over.  wide_extreme gives the
 // largest magnitude, wide_fields by the width the 32-bit fields or the packed fields of a
 // wide row.
+constexpr uint32_t kWide = 1, kGone = 2;
 template <typename T, bool FULL, uint32_t RT, typename Diff>
-__device__ __forceinline__ bool wide_residuals(const RowPass<T, RT> &P, uint64_t *slots, uint32_t &rm, Diff diff) {
+__device__ __forceinline__ uint32_t wide_residuals(const RowPass<T, RT> &P, uint64_t *slots, uint32_t &rm, Diff diff) {
   constexpr uint32_t V = 16 / sizeof(T);
   int32_t mx = 0, mn = 0, r[4];
   uint32_t bad = 0;
-  for_slots<T, FULL, 8 / V>(P.rowa, P.cnt, [&](uint32_t i, const T *y) {
+  bool up0;
+  const uint64_t d0 = diff(staged_value<T>(P.rowa, 0), 0, up0);
+  if (__all_sync(0xffffffffu, d0 >> 31 && (FULL || P.cnt))) {
+    bad = kWide;
+  } else {
+    for_slots<T, FULL, 8 / V>(P.rowa, P.cnt, [&](uint32_t i, const T *y) {
 #pragma unroll
-    for (uint32_t j = 0; j < V; ++j) {
-      bool up;
-      uint64_t d = diff(y[j], V * i + j, up);
-      if (!FULL && V * i + j >= P.cnt) d = 0;
-      bad |= (uint32_t)(d >> 32) | ((uint32_t)d & 0x80000000u);
-      if (sizeof(T) == 4) bad |= (uint32_t)(up && d == 0);  // a magnitude that is 0 mod 2^32 keeps its sign bit
-      const int32_t v = up ? (int32_t)(uint32_t)d : -(int32_t)(uint32_t)d;
-      mx = max(mx, v);
-      mn = min(mn, v);
-      r[(V * i + j) & 3u] = v;
-    }
-    if (V == 4 || (i & 1u)) put_slot(P.rowa, V == 4 ? i : i >> 1, r);
-  });
+      for (uint32_t j = 0; j < V; ++j) {
+        bool up;
+        uint64_t d = diff(y[j], V * i + j, up);
+        if (!FULL && V * i + j >= P.cnt) d = 0;
+        bad |= (uint32_t)(d >> 32) | ((uint32_t)d & 0x80000000u);
+        if (sizeof(T) == 4) bad |= (uint32_t)(up && d == 0);  // a magnitude that is 0 mod 2^32 keeps its sign bit
+        const int32_t v = up ? (int32_t)(uint32_t)d : -(int32_t)(uint32_t)d;
+        mx = max(mx, v);
+        mn = min(mn, v);
+        r[(V * i + j) & 3u] = v;
+      }
+      if (V == 4 || (i & 1u)) put_slot(P.rowa, V == 4 ? i : i >> 1, r);
+    });
+    bad = kGone | (bad ? kWide : 0u);
+  }
   rg_reduce3<true>(P.g, mx, mn, bad, slots);
   rm = max((uint32_t)mx, (uint32_t)(-mn));
-  return !bad;
+  return bad & kWide ? bad : 0u;
 }
 template <typename T, bool FULL, uint32_t RT, typename Diff>
 __device__ __forceinline__ uint64_t wide_extreme(const RowPass<T, RT> &P, Diff diff) {
@@ -891,15 +914,10 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
   constexpr uint32_t S = sizeof(T), TB = 8 * S, V = 16 / S;
   const RowGroup<RT> &g = P.g;
   const uint32_t len = P.len, cnt = P.cnt, p0 = 32 * g.rank;
-  // (the values have been replaced by residuals when the width says raw)
+  // The values once more, after residuals have taken their place (every thread of the group).
   auto restage = [&]() {
-    const T *src = reinterpret_cast<const T *>(a.values) + b * a.bs + p0;
-    for (uint32_t j = 0; j < 32; ++j) {
-      const T y = j < cnt ? __ldg(src + j) : (T)0;
-      const uint32_t at = (P.rowa ^ ((j / V) << 4)) + (j % V) * S;
-      sts_u32(at, (uint32_t)y);
-      if (S == 8) sts_u32(at + 4, (uint32_t)((uint64_t)y >> 32));
-    }
+    stage_rows<T>(g, sb, reinterpret_cast<const T *>(a.values) + b * a.bs, len);
+    g.sync_apart();
   };
   auto finish_width = [&](uint32_t l) {  // the width a block of this codec is written with
     if (l > TB) l = TB;
@@ -931,7 +949,7 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
     C.m0 = model[0];
     C.m1 = model[1];
     C.m2 = model[2];
-    bool coded = false;
+    bool coded = false, wide = false;
     uint64_t *wide_slots = P.slots[1];
     if constexpr (CODEC == kLinear) {
       // ---- midpoint shift (piecewise_fix_integer_template.h:36-46) ----
@@ -970,6 +988,8 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
           dmax = (int64_t)(ux ^ (1ull << 63));
           dmin = (int64_t)(~un ^ (1ull << 63));
           small = dmax >= dmin && (uint64_t)(dmax - dmin) < (1ull << 30);
+          // half of a span this large has no 32-bit residual (u64), or makes the block raw (u32)
+          wide = dmax >= dmin && (uint64_t)dmax - (uint64_t)dmin >= (S == 8 ? (1ull << 32) : (1ull << 31)) + 16;
           const int64_t mid = (int64_t)((uint64_t)dmax + (uint64_t)dmin);
           C.m0 = __dadd_rn(C.m0, __dmul_rn(__ll2double_rn(mid), 0.5));
         }
@@ -995,8 +1015,11 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
           const uint64_t d = up ? v - (uint64_t)p : (uint64_t)p - v;
           return S == 4 ? d & 0xffffffffull : d;
         };
-        uint32_t rm;
-        const bool fits = wide_residuals<T, FULL>(P, wide_slots, rm, diff);
+        uint32_t rm = 0, state = kWide;
+        // (a warp of blocks known to be wide does not try; their values are still there)
+        const bool known = __all_sync(0xffffffffu, wide);
+        if (!known) state = wide_residuals<T, FULL>(P, wide_slots, rm, diff);
+        const bool fits = !state;
         if (fits) {
           C.l = finish_width(rm ? bits_of(rm) + 1 : 0);
           if (S == 4 && C.l == TB) restage();
@@ -1004,11 +1027,11 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
         if (!__all_sync(0xffffffffu, fits)) {  // the same again, from the values
           uint64_t rmax = 0, none = 0;
           if (!fits) {
-            restage();
+            if (state & kGone) restage();
             rmax = wide_extreme<T, FULL>(P, diff);
           }
           __syncwarp();
-          rg_max<false>(g, rmax, none, wide_slots == P.slots[1] ? P.slots[0] : P.slots[1]);
+          rg_max<false>(g, rmax, none, known ? wide_slots : wide_slots == P.slots[1] ? P.slots[0] : P.slots[1]);
           if (!fits) {
             C.l = finish_width(rmax ? bits_of(rmax) + 1 : 0);
             if (C.l < TB) wide_fields<T, FULL>(P, C.l, diff);
