@@ -224,15 +224,29 @@ __global__ void __launch_bounds__(32) seq_fit_ring_kernel(const T *__restrict__ 
 // Columns of at least this many blocks take the fits from the kernels below, which read the
 // values once more but at up to 6 TB/s, and leave the row encoder without its own.  A short
 // column's fit kernel is bound by one block's chain of dependent additions (71 us for 4096
-// values, one block or thousands), which the row encoder does not have.  u64, us with the fit
-// kernel / with the fits inside:
-//   blocks of 4096 values, LeCo:   4096: 147 / 114   8192: 200 / 207   12288: 257 / 298   24576: 485 / 599
-//   blocks of 1000 values, LeCo:   4096:  52 /  42   8192:  73 /  69   12288:  99 / 112   24576: 168 / 199
-//   blocks of 4096 values, poly2:  4096: 154 / 143   8192: 218 / 284   12288: 278 / 431   24576: 537 / 883
-//   blocks of 1000 values, poly2:  4096:  53 /  51   8192:  73 /  91   12288:  98 / 143   24576: 183 / 279
+// values, one block or thousands), which the row encoder does not have; its own fit costs more
+// where a block's CTA is large (fewer fit an SM with the fit's tables).  us with the fit kernel /
+// with the fits inside:
+//   u64 LeCo   1000 values:  4096:  52 /  42   8192:  73 /  69  12288:  99 / 112  24576: 168 / 199
+//              4096 values:  4096: 147 / 114   8192: 200 / 207  12288: 257 / 298  24576: 485 / 599
+//              5000 values:  4000: 198 / 165   5000: 221 / 209   6000: 245 / 257   8000: 280 / 340
+//              8192 values:  5000: 300 / 257   6000: 330 / 306   8000: 372 / 398
+//              9000 values:  3000: 289 / 257   4000: 317 / 339   5000: 349 / 416
+//             12000 values:  3000: 380 / 302   4000: 415 / 394   5000: 466 / 487
+//             16384 values:  3000: 559 / 472   4000: 626 / 615   5000: 716 / 764
+//   u64 poly2  1000 values:  4096:  53 /  51   8192:  73 /  91  12288:  98 / 143
+//              4096 values:  4096: 154 / 143   8192: 218 / 284  12288: 278 / 431
+//              5000 values:  2000: 161 / 125   3000: 189 / 180   4000: 210 / 244
+//             12000 values:  1000: 293 / 194   2000: 341 / 379   3000: 387 / 562
+//             16384 values:  2000: 482 / 394   3000: 553 / 574   4000: 621 / 757
+//   u32 poly2  9000 values:  2000: 225 / 170   3000: 267 / 261   4000: 307 / 344
+//             16384 values:  3000: 412 / 349   4000: 457 / 458   5000: 506 / 560
 // u32 LeCo columns keep the fits inside at every size: their sums seldom reach 2^53, so the
 // row encoder takes them from its scan.
-constexpr uint64_t kSeqFitBlocks = 8192, kSeqFitBlocksPoly = 5120;
+static uint64_t seq_fit_blocks(int codec, uint32_t bs) {
+  if (codec == kLinear) return bs > 8192 ? 4096 : bs > 4096 ? 6144 : 8192;
+  return bs > 4096 ? 2560 : 5120;
+}
 // The sequential fits of a column's blocks into L.seq_models (CODEC: kLinear, also for the
 // legacy codec, or kPoly2).
 template <typename T, int CODEC>
@@ -260,7 +274,7 @@ int launch_encode(int codec, int s, const EncodeLaunch &L, cudaStream_t st) {
   for (int i = 0; i < 10; ++i) a.polyX[i] = L.polyX[i];
   if (codec != kLegacy) {
     const bool ref = L.seq_models != nullptr;
-    if (ref && (codec == kLinear ? s == 8 && L.nb >= kSeqFitBlocks : L.nb >= kSeqFitBlocksPoly)) {  // (FOR and Delta: never ref)
+    if (ref && (codec != kLinear || s == 8) && L.nb >= seq_fit_blocks(codec, L.bs)) {  // (FOR and Delta: never ref)
       if (codec == kLinear) launch_seq_fit<uint64_t, kLinear>(L, st);
       else if (s == 8) launch_seq_fit<uint64_t, kPoly2>(L, st);
       else launch_seq_fit<uint32_t, kPoly2>(L, st);

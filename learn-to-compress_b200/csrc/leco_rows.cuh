@@ -44,26 +44,35 @@ namespace leco {
 constexpr double kExactSum = 9007199254740992.0;  // 2^53
 constexpr int32_t kNoEffect = -32768;
 
-// Threads per block: a power of two >= the block's rows.
+// Threads per block where blocks share a CTA: a power of two >= the block's rows.
 __host__ __device__ inline uint32_t rows_threads(uint32_t bs) {
   const uint32_t rows = (bs + 31) / 32;
   uint32_t r = 8;
   while (r < rows) r <<= 1;
   return r;
 }
+// The same for a column of its own: a block of more than 64 rows has its CTA for itself, of as
+// many warps as its rows need where that lets more CTAs onto an SM than the next power of two
+// (of 224 threads there are as few as of 256; of 416 and 448 two fit where the fit is not in the
+// encoder, if the codec needs no more than 72 registers).  60M u64 values, power of two / this,
+// us: FOR in blocks of 9000 (283 rows) 418 / 217, LeCo with the exact fit in blocks of 5000
+// 472 / 376, of 9000 658 / 356.
+__host__ __device__ inline uint32_t column_rows_threads(int codec, uint32_t bs) {
+  const uint32_t rows = (bs + 31) / 32, r = (rows + 31) / 32 * 32, most = codec == kPoly2 ? 384u : 448u;
+  return rows <= 64 ? rows_threads(bs) : r == 224 ? 256u : r > most ? 512u : r;
+}
+constexpr uint32_t kWholeCta = 0xffffffffu;  // RT of a block's group that is the CTA, of any number of warps
 __host__ __device__ constexpr int rows_sums(int codec) { return codec == kLinear ? 2 : codec == kPoly2 ? 3 : 0; }
 
-// Shared memory of one CTA of nt threads in groups of R.
+// Shared memory of one CTA of nt threads in groups of R; from tab on for the reference's fit
+// in the encoder only (`total` with it, `tab` without).
 struct RowsLayout {
-  uint32_t tab, base, mask, wtot, red, hdr, model, size, goff, count, total;
+  uint32_t wtot, red, hdr, model, size, goff, count, tab, base, mask, total;
 };
 __host__ __device__ constexpr RowsLayout rows_layout(uint32_t nt, uint32_t R, uint32_t s, uint32_t ns) {
   RowsLayout L{};
   const uint32_t ng = nt / R, nw = nt / 32;
   uint32_t o = nt * 32 * s;                 // rows of 32 values
-  L.tab = o;   o += ns * nt * 8;            // [ns][nt]: a row's effect (four int16) or its run's (two int32)
-  L.base = o;  o += ns * (nt + ng) * 8;     // u64 [ns][groups * (R + 1)]: the rows' approximate starts
-  L.mask = o;  o += ns * nw * 8;            // uint2 [ns][warps]: rows to walk, uncertain rows
   L.wtot = o;  o += 3 * nw * 8;             // double [3][warps]
   L.red = o;   o += 2 * 2 * nw * 8;         // u64 [2][2][warps]
   L.hdr = o;   o += ng * 32;                // u64 [groups][4]: header bytes
@@ -71,30 +80,34 @@ __host__ __device__ constexpr RowsLayout rows_layout(uint32_t nt, uint32_t R, ui
   L.size = o;  o += ng * 8;                 // u64 [groups]
   L.goff = o;  o += ng * 8;                 // u64 [groups]
   L.count = o; o += 8;                      // u32: groups whose size is known
+  L.tab = o;   o += ns * nt * 8;            // [ns][nt]: a row's effect (four int16) or its run's (two int32)
+  L.base = o;  o += ns * (nt + ng) * 8;     // u64 [ns][groups * (R + 1)]: the rows' approximate starts
+  L.mask = o;  o += ns * nw * 8;            // uint2 [ns][warps]: rows to walk, uncertain rows
   L.total = o;
   return L;
 }
 
 // A thread's place: `rank` in its group of R threads (= its row of the block).  RT: the group
-// size when it is fixed at compile time, else 0.
+// size when it is fixed at compile time, kWholeCta when it is the CTA's, else 0 (a power of two).
 template <uint32_t RT>
 struct RowGroup {
   uint32_t nt, Rd, gi, rank, row;  // row: the row's place in shared memory (threadIdx.x)
   uint32_t lane, gl;               // lane, lane among the group's lanes of this warp
   uint32_t warp, w0;               // this warp, the group's first warp
-  __device__ __forceinline__ uint32_t R() const { return RT ? RT : Rd; }
+  static constexpr bool whole = RT == kWholeCta;
+  __device__ __forceinline__ uint32_t R() const { return RT && !whole ? RT : Rd; }
   __device__ __forceinline__ uint32_t rl() const { return RT >= 32 ? 32u : RT ? RT : (Rd < 32 ? Rd : 32u); }
-  __device__ __forceinline__ uint32_t nw() const { return RT >= 32 ? RT / 32 : RT ? 1u : (Rd < 32 ? 1u : Rd / 32); }
+  __device__ __forceinline__ uint32_t nw() const { return whole ? Rd / 32 : RT >= 32 ? RT / 32 : RT ? 1u : (Rd < 32 ? 1u : Rd / 32); }
   __device__ __forceinline__ explicit RowGroup(uint32_t R) {
     Rd = R;
     nt = blockDim.x;
     row = threadIdx.x;
-    rank = threadIdx.x & (this->R() - 1);
+    rank = whole ? threadIdx.x : threadIdx.x & (this->R() - 1);
     gi = RT ? threadIdx.x / (RT ? RT : 1u) : threadIdx.x >> (31 - __clz((int)R));
     lane = threadIdx.x & 31;
     gl = lane & (rl() - 1);
     warp = threadIdx.x >> 5;
-    w0 = nw() == 1 ? warp : gi * nw();
+    w0 = whole ? 0u : nw() == 1 ? warp : gi * nw();
   }
   __device__ __forceinline__ void sync() const {
     // Barriers by constant numbers: the warps of a group may wait at different places of the
@@ -178,25 +191,32 @@ __device__ __forceinline__ void rg_max(const RowGroup<RT> &g, uint64_t &a, uint6
     }
   }
 }
-// Sum of 128-bit values over the group; `slots`: two u64 [warps] rows.  The callers' next
-// use of the same slots must come after a group barrier.
-template <uint32_t RT>
-__device__ __forceinline__ u128 rg_sum128(const RowGroup<RT> &g, u128 v, uint64_t *slots) {
-  for (uint32_t m = 1; m < g.rl(); m <<= 1) {
-    const uint64_t lo = shfl_xor_u64((uint64_t)v, m), hi = shfl_xor_u64((uint64_t)(v >> 64), m);
-    v += ((u128)hi << 64) | lo;
-  }
-  if (g.nw() == 1) return v;
+// Sums of N 128-bit values over the group; `slots`: 2 * N u64 [warps] rows that may still be
+// read.  The callers' next use of them must come after a group barrier.
+template <int N, uint32_t RT>
+__device__ __forceinline__ void rg_sums128(const RowGroup<RT> &g, u128 (&v)[N], uint64_t *slots) {
+#pragma unroll
+  for (int s = 0; s < N; ++s)
+    for (uint32_t m = 1; m < g.rl(); m <<= 1) {
+      const uint64_t lo = shfl_xor_u64((uint64_t)v[s], m), hi = shfl_xor_u64((uint64_t)(v[s] >> 64), m);
+      v[s] += ((u128)hi << 64) | lo;
+    }
+  if (g.nw() == 1) return;
   const uint32_t nws = g.nt >> 5;
   g.sync();
   if (g.lane == 0) {
-    slots[g.warp] = (uint64_t)v;
-    slots[nws + g.warp] = (uint64_t)(v >> 64);
+#pragma unroll
+    for (int s = 0; s < N; ++s) {
+      slots[2 * s * nws + g.warp] = (uint64_t)v[s];
+      slots[(2 * s + 1) * nws + g.warp] = (uint64_t)(v[s] >> 64);
+    }
   }
   g.sync();
-  v = 0;
-  for (uint32_t w = g.w0; w < g.w0 + g.nw(); ++w) v += ((u128)slots[nws + w] << 64) | slots[w];
-  return v;
+#pragma unroll
+  for (int s = 0; s < N; ++s) {
+    v[s] = 0;
+    for (uint32_t w = g.w0; w < g.w0 + g.nw(); ++w) v[s] += ((u128)slots[(2 * s + 1) * nws + w] << 64) | slots[2 * s * nws + w];
+  }
 }
 
 // ---- rows in shared memory -------------------------------------------------------
@@ -234,7 +254,7 @@ __device__ __forceinline__ void stage_rows(const RowGroup<RT> &g, uint32_t sb, c
     if (RT >= 64 && nc == g.R() * SL) {  // a block of R full rows
 #pragma unroll
       for (uint32_t i = 0; i < SL; ++i) {
-        const uint32_t q = g.rank + i * RT;
+        const uint32_t q = g.rank + i * g.R();
         cp_async16(row_at<T>(sb, r0 + q / SL) ^ ((q % SL) << 4), src + (size_t)q * V);
       }
     } else {
@@ -614,12 +634,13 @@ __device__ __forceinline__ void rows_fit(const RowGroup<RT> &g, uint32_t len, ui
     });
     const u128 sy = ((u128)shi << 32) + slo, sj = ((u128)thi << 32) + tlo, sq = ((u128)qhi << 32) + qlo;
     const uint64_t i0 = 32ull * g.rank;
-    uint64_t *slots = reinterpret_cast<uint64_t *>(smem + L.red);
-    const u128 m0 = rg_sum128(g, sy, slots), m1 = rg_sum128(g, sy * i0 + sj, slots);
-    u128 m2 = 0;
-    if (NS == 3) m2 = rg_sum128(g, sy * (i0 * i0) + sj * (2 * i0) + sq, slots);
+    u128 m[NS];
+    m[0] = sy;
+    m[1] = sy * i0 + sj;
+    if constexpr (NS == 3) m[2] = sy * (i0 * i0) + sj * (2 * i0) + sq;
+    rg_sums128<NS>(g, m, reinterpret_cast<uint64_t *>(smem + L.wtot));  // (wtot and red together)
     if (g.rank == 0 && any)
-      store_seq_model<CODEC>(model, u128_to_double(m0), u128_to_double(m1), u128_to_double(m2), len, bs, polyX);
+      store_seq_model<CODEC>(model, u128_to_double(m[0]), u128_to_double(m[1]), u128_to_double(m[NS - 1]), len, bs, polyX);
   }
   g.sync();
 }
@@ -1213,18 +1234,18 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
 // barriers, so its width matters both ways: 24.6M u32 FOR / Delta values, us: windows of 128
 // words 47 / 48, 256 42 / 44, 512 41 / 44, 1024 50 / 51; one warp stepping over 256 words 47 / 50.
 constexpr uint32_t kPubWindow = 512;
-template <uint32_t NT>
+template <uint32_t NT>  // at most NT threads
 __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, uint32_t *error, uint8_t *smem,
                                               uint32_t spin_limit = kSpinLimit) {
   constexpr uint32_t NW = NT / 32, kPubWords = kPubWindow / NT;
   uint64_t *wsum = reinterpret_cast<uint64_t *>(smem);                // [2][NW]
   uint32_t *wfirst = reinterpret_cast<uint32_t *>(smem + 2 * NW * 8);  // [2][NW]
-  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5, window = kPubWords * blockDim.x;
   uint64_t run = 0, j = 0;  // inclusive prefix before item j
   uint32_t spins = 0, par = 0;
   while (j < items) {
     uint64_t v[kPubWords];
-    uint32_t first = NT * kPubWords;  // this thread's first unpublished place
+    uint32_t first = window;  // this thread's first unpublished place
 #pragma unroll
     for (uint32_t k = 0; k < kPubWords; ++k) {
       const uint64_t idx = j + kPubWords * t + k;
@@ -1247,13 +1268,14 @@ __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, 
     if (lane == 31) wsum[par * NW + warp] = incl;
     if (lane == 0) wfirst[par * NW + warp] = first;
     __syncthreads();  // (the two halves of the scratch alternate, so one barrier a step is enough)
-    uint32_t n = NT * kPubWords;
+    uint32_t n = window;
     uint64_t before = run + incl - own;
 #pragma unroll
-    for (uint32_t w = 0; w < NW; ++w) {
-      n = min(n, wfirst[par * NW + w]);
-      if (w < warp) before += wsum[par * NW + w];
-    }
+    for (uint32_t w = 0; w < NW; ++w)
+      if (w < nw) {
+        n = min(n, wfirst[par * NW + w]);
+        if (w < warp) before += wsum[par * NW + w];
+      }
     // the published run is items j .. j + n - 1: words past n (in any thread) are left
     uint64_t last = 0;
     bool has_last = false;
@@ -1328,9 +1350,13 @@ __device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t i
   stage_rows<T>(g, sb, reinterpret_cast<const T *>(a.values) + b * a.bs, len);
   __syncthreads();
   RowCoded C{};
-  // (the two ways meet at the same barriers: the warps of a block may differ)
+  // (the two ways meet at the same barriers: the warps of a block may differ.  With a model they
+  // do not: the last rows' warp then held up all others, and both forms of the passes in use at
+  // once cost more than the masks of the one -- 60M u64, exact fit, blocks of 3000: LeCo 439 us,
+  // 390 so; poly2 671, 518.  FOR and Delta are faster with both.)
   uint64_t *status = alone ? nullptr : a.status + item;
-  if (__all_sync(0xffffffffu, P.cnt == 32)) encode_rows_passes<T, CODEC, true>(a, P, ref, sb, smem, L, b, C, status);
+  constexpr bool kModel = CODEC == kLinear || CODEC == kPoly2;
+  if (__all_sync(0xffffffffu, kModel ? len == 32 * R : P.cnt == 32)) encode_rows_passes<T, CODEC, true>(a, P, ref, sb, smem, L, b, C, status);
   else encode_rows_passes<T, CODEC, false>(a, P, ref, sb, smem, L, b, C, status);
   const uint32_t l = C.l;
   const bool raw = l == TB;
