@@ -32,7 +32,8 @@ __global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 4 ? 6 : 0
 
 // Small blocks: one warp per block, eight blocks per CTA.
 template <typename T, int CODEC>
-__global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 8 ? 5 : 0) decode_kernel_warp(DecodeLaunch a, uint64_t nblk) {
+__global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 8 ? 5 : 0)
+    decode_kernel_warp(DecodeLaunch a, uint64_t nblk) {
   const uint64_t i = (uint64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (i < nblk) decode_block<T, CODEC, 32>(a, a.first / a.bs + i);
 }
@@ -81,15 +82,17 @@ struct StageMeta {
 // blockIdx.x + gridDim.x, ...; thread 0 stages the next block's image (header +
 // packed body) into the other half of a double buffer with one cp.async.bulk
 // while the CTA decodes the current one out of shared memory.  Blocks that do
-// not fit the buffer and wide (l > 32) blocks take the direct path.  Delta blocks
-// run the row scan (delta_tiles), which synchronises the CTA, so for Delta the
-// CTA decodes a block only when every thread's wait succeeded.
+// not fit the buffer and wide (l > 32) blocks take the direct path.  Delta has a
+// kernel of its own below; its sums run the row scan (delta_tiles), which synchronises
+// the CTA, so for Delta the CTA takes a block only when every thread's wait succeeded.
 // SUM: the compressed-domain sum instead -- the values are added up, not stored,
 // and each CTA adds its total to *d_sum once.  (u32 Delta: 40 registers, six CTAs per SM; with
 // 64 the sums of 60M random values in blocks of 1000 / 8192 took 154 / 218 us instead of
 // 135 / 157.)
 template <typename T, int CODEC, bool SUM = false>
-__global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 4 ? 6 : 0) decode_staged_kernel(DecodeLaunch a, uint32_t bufcap, uint64_t *d_sum = nullptr) {
+__global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 4 ? 6 : 0)
+    decode_staged_kernel(DecodeLaunch a, uint32_t bufcap, uint64_t *d_sum = nullptr) {
+  static_assert(CODEC != kDelta || SUM, "bulk Delta decode is decode_delta_kernel");
   constexpr int S = sizeof(T);
   extern __shared__ __align__(128) uint8_t stage[];
   __shared__ __align__(8) uint64_t bar[2];
@@ -155,15 +158,11 @@ __global__ void __launch_bounds__(256, CODEC == kDelta && sizeof(T) == 4 ? 6 : 0
         h.base = w;
         h.body_bit = (uint64_t)(m.hoff + Hdr<CODEC, S>::bytes) * 8;
         const uint64_t *sw = reinterpret_cast<const uint64_t *>(sb);
-        if (SUM) {
-          delta_tiles<T, 256, true>(sw, h, len, 0, len, [&](uint32_t k0, const auto *v) {
-  #pragma unroll
-            for (int j = 0; j < kDeltaSpan; ++j)
-              if (k0 + j < len) acc += (uint64_t)(T)v[j];
-          });
-        } else {
-          delta_tiles<T, 256, true>(sw, h, len, 0, len, DeltaStore<T>{out, base, 0, len});
-        }
+        delta_tiles<T, 256, true>(sw, h, len, 0, len, [&](uint32_t k0, const auto *v) {
+#pragma unroll
+          for (int j = 0; j < kDeltaSpan; ++j)
+            if (k0 + j < len) acc += (uint64_t)(T)v[j];
+        });
       } else {
         BlockHdr h;
         h.l = l;
@@ -578,7 +577,7 @@ static void run_decode(const DecodeLaunch &L, cudaStream_t st) {
     else decode_kernel<T, CODEC><<<(unsigned)nblk, 256, 0, st>>>(L);
     return;
   }
-  // +128: field reads may run past a full buffer, a Delta span's by up to 68 bytes
+  // +128: field reads may run past a full buffer, a Delta span's (nine words) by up to 36 bytes
   const int smem = 2 * kStageBuf + 128;
   if constexpr (CODEC == kDelta) {
     const LaunchInfo i = launch_info<decode_delta_kernel<T>>(256, smem);
