@@ -279,11 +279,11 @@ typedef struct leco_column_desc {
   int32_t codec;       /* LINEAR, FOR, DELTA or POLY2                          */
   int32_t dtype;       /* LECO_U32 or LECO_U64                                 */
   uint32_t block_size; /* values per block, 1..16384                           */
-  uint16_t group_threads; /* batch engine: threads per block, 32/64/128/256;
+  uint16_t group_threads; /* batch decoder: threads per block, 32/64/128/256;
                              0 = 32 for blocks of <= 512 values, else 256       */
-  uint16_t unroll;     /* batch engine: unroll depth 1/2/4 (0 = 2): the decoder
-                          writes `unroll` 16-byte chunks per thread step, the u64
-                          LeCo encoder keeps 2*unroll 16-byte loads in flight   */
+  uint16_t unroll;     /* batch decoder: unroll depth 1/2/4 (0 = 2): `unroll`
+                          16-byte chunks written per thread step.  (The encoder
+                          takes one thread per 32 values whatever these say.)   */
   uint64_t n;          /* values in the column                                 */
   const void *d_values;/* encode input (n values)                              */
   void *d_out;         /* decode output (n values); may be NULL if never decoded */
@@ -298,16 +298,17 @@ typedef struct leco_batch leco_batch; /* opaque */
 /* Builds a batch over ncols column descriptors (copied).  Allocates the device
  * descriptor table and the batch workspace (the only allocations of the batch
  * engine); sizes the persistent grids so every CTA is resident.  A column's
- * work items hold 256/group_threads blocks, one per group of a 256-thread CTA;
- * an item's shared memory (enc_smem per block x blocks per item) must stay
- * within 200 KB, else LECO_ERR_ARG.  The committed autotune table gives
- * block_size, group_threads and unroll per column shape. */
+ * decoder items hold 256/group_threads blocks, one per group of a 256-thread CTA.
+ * The values of 256/group_threads blocks, with about 1.3 KB and 4 bytes per 32
+ * values for each block, must stay within 200 KB, else LECO_ERR_ARG.  The
+ * committed autotune table gives block_size, group_threads and unroll per column
+ * shape. */
 int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mode, leco_batch **out);
 int leco_batch_destroy(leco_batch *b);
 uint64_t leco_batch_total_blocks(const leco_batch *b);
 /* Encodes every block of every column with one persistent launch pulling
- * (column, block) items from an atomic work queue (plus the sequential-fit pass
- * for reference-fit columns that need it). */
+ * (column, block) items from an atomic work queue, fits included; columns with
+ * blocks of more than 8192 values have a second launch of their own. */
 int leco_batch_encode(leco_batch *b, leco_stream_t stream);
 /* Decodes every column into its d_out (aligned to the column's value size) with one
  * persistent launch. */

@@ -6,19 +6,18 @@ length bucket):
 * values per block (256 .. 16384): the size that gives the smallest encoded
   column; among sizes within 0.5 % of that, the one with the shortest measured
   single-column encode+decode time;
-* threads per block G (32, 64, 128, 256): the batch engine runs 256/G blocks
+* threads per block G (32, 64, 128, 256): the batch decoder runs 256/G blocks
   of a work item side by side in one 256-thread CTA, one group of G threads per
   block (G = 32: one warp per block);
-* unroll depth U (1, 2, 4): the decoder writes U 16-byte chunks per thread
-  step; the u64 LeCo encoder keeps 2U 16-byte loads in flight per thread.
+* unroll depth U (1, 2, 4): the decoder writes U 16-byte chunks per thread step.
 
-G and U are chosen by timing a batch pass (encode + decode, replayed as a CUDA
-graph) over a batch of columns of that shape for every feasible (G, U) -- a
-combination is feasible when the 256/G blocks of an item fit in the ~72 KB of
-shared memory that keep three CTAs per SM (the batch encode kernel sizes every
-CTA for the largest item) -- keeping the engine's default
-(G = 32 for blocks of <= 512 values, else 256; U = 2) unless another is more
-than 2 % faster.  The table is produced on a B200 by
+The batch encoder takes one thread per 32 values and neither G nor U.  The
+committed table was measured when it took both: G and U are chosen by timing a
+batch pass (encode + decode, replayed as a CUDA graph) over a batch of columns of
+that shape for every feasible (G, U), keeping the engine's default (G = 32 for
+blocks of <= 512 values, else 256; U = 2) unless another is more than 2 % faster.
+A combination is feasible when the values of 256/G blocks stay within ~72 KB, the
+limit of that measurement.  The table is produced on a B200 by
 ``python -m leco_b200.autotune`` (import name of this package) and committed as
 ``autotune_table.json``; at run time ``pick`` looks a column up, after
 ``classify`` has put it in a family from a sample of its values.
@@ -39,21 +38,20 @@ GROUPS = (32, 64, 128, 256)
 UNROLLS = (1, 2, 4)
 FAMILIES = ("linear", "step", "walk", "uniform")
 LEN_BUCKETS = tuple(1 << k for k in range(10, 23, 2))  # 1K .. 4M
-BATCH_MAX_SMEM = 200 * 1024  # shared memory one work item may use (leco_batch.cu)
-# The batch encode kernel takes the largest item's shared memory for every CTA, so
-# the tuner keeps each choice within what the default launch already needs for the
-# largest blocks (16384 u32 / 8192 u64 values, ~69 KB): three CTAs per SM.
+BATCH_MAX_SMEM = 200 * 1024  # what leco_batch_create accepts for a (block size, G)
+# The tuner keeps each choice within what G = 256 has for the largest blocks it tries
+# (16384 u32 / 8192 u64 values, ~69 KB).
 TUNE_MAX_SMEM = 72 * 1024
 
 
 def max_block(dtype_bytes: int) -> int:
-    """Largest block the batch engine stages in shared memory at 3+ CTAs/SM."""
+    """Largest block the tuner tries: what the batch encoder stages at three CTAs per SM (u64)."""
     return 16384 if dtype_bytes == 4 else 8192
 
 
 def enc_smem_bytes(bs: int, s: int) -> int:
-    """Encoder shared memory of one block (enc_smem_bytes in leco_encode.cuh),
-    rounded to 16 bytes as the batch engine lays out its groups."""
+    """A block's share in the limit on (block size, G): enc_smem_bytes in leco_encode.cuh, rounded
+    to 16 bytes."""
     b = 1152 + ((bs // 32 + 9) * 4 + 15) // 16 * 16 + (bs + 31) // 32 * 32 * s + 16
     return (b + 15) // 16 * 16
 

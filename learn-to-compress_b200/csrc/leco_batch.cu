@@ -13,7 +13,10 @@
 // look-back (byte offsets, one word per item) only ever waits on items that are already
 // being processed.  The reference's sequential fits are part of the encoder item
 // (rows_fit): as a pass of their own, one lane per block, they took 606 of the 949 us of an
-// encode + decode pass over 20 columns of 64K-4M values; the whole pass takes 160 us now.
+// encode + decode pass over 20 columns of 64K-4M values; the whole pass takes 162 us now.
+// Every CTA of an encode launch has the shared memory of the batch's largest item: three CTAs
+// per SM with LeCo, FOR and Delta columns, two for all of them when one is u64 degree-2 in large
+// blocks.  The encode kernel holds every codec's encoder in 80 registers and spills some of them.
 //
 // The reference has no counterpart: its drivers loop over blocks of one column
 // (experiments/leco_int_fix_template.cpp:111-127, :145-153).  The per-column
@@ -49,7 +52,7 @@ struct leco_batch {
 
 namespace {
 
-// Shared memory one work item may take (the CTA limit is 227 KB).
+// What a column's (block size, group_threads) may ask for: see the rule in leco_batch_create.
 constexpr uint32_t kBatchMaxSmem = 200 * 1024;
 
 // The most shared memory an encoder item can take (any codec, value type and block size).  A
@@ -137,7 +140,9 @@ int leco_batch_create(const leco_column_desc *h_cols, uint32_t ncols, int fit_mo
       return berr(LECO_ERR_ARG, "leco_batch_create: column " + std::to_string(i) +
                                     ": group_threads must be 0, 32, 64, 128 or 256 and unroll 0, 1, 2 or 4");
     }
-    // (the limit of group_threads: a group's values, held once for each group of 256 threads)
+    // The rule for group_threads of the interface: its blocks' values, one slice for each group of
+    // a 256-thread CTA, within 200 KB.  (Neither kernel lays its items out so: the encoder's follow
+    // the block size alone, the decoder's need no shared memory.)
     const uint32_t slice = (enc_smem_bytes(c.block_size, (uint32_t)c.dtype) + 15) / 16 * 16;
     const uint32_t item_smem = slice * (256 / d.group);
     if (item_smem > kBatchMaxSmem) {

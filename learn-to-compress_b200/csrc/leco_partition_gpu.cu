@@ -304,10 +304,13 @@ __global__ void __launch_bounds__(kPartThreads) partition_kernel(PartitionArgs a
 // absorbed is skipped.  Phase 2 keeps 16-bit starts, sizes and pair sizes; a pair's size is
 // computed again only when one of the two segments has changed.
 // Bound by latency: phase 1 is one warp's, phase 2 mostly sums of the fits.  Shared memory:
-// 14 bytes a value, eight CTAs per SM for blocks of 2000 values.  10M values, 5000 blocks of
+// 14 bytes a value and 3 KB, seven CTAs per SM for blocks of 2000 values, one for blocks of 8000.  10M values, 5000 blocks of
 // 2000, partition and encode: 43.7 ms with a thread per block, 4.47 ms with one warp per
 // block that scanned every class over all positions, 1.86 ms now.
-constexpr uint32_t kPartCtaMax = 8000;   // sizes fit 16 bits, shared memory fits an SM twice
+// The longest block of a CTA: starts and sizes fit 16 bits (a raw segment takes 8 bytes a value
+// and 5).  2M values in blocks of 8000 / 8001: 2.1 ms / 146 ms, so the limit is the form's, not
+// the point where the other kernel wins.
+constexpr uint32_t kPartCtaMax = 8000;
 // A column of many short coarse blocks keeps the thread per block: a CTA's barriers and list
 // set-up take about 5 ns a block when all SMs are full, whatever its size, while a thread's
 // chain shortens with it.  CTA time over thread time, regime-switching column / random values:
@@ -916,7 +919,7 @@ int leco_varlen_partition_device(const uint64_t *d_values, uint64_t n, uint32_t 
     if (se == cudaSuccess) se = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, partition_cta_kernel, 32 * kPartWarps, smem);
     if (se != cudaSuccess)
       return record_error(LECO_ERR_CUDA, std::string("leco_varlen_partition_device: ") + cudaGetErrorString(se));
-    // a CTA's scratch (16 bytes a value) lies in its slot's segment list (48 bytes a value): no more CTAs than slots
+    // a CTA's scratch (16 bytes a value) lies in its slot's segment list (40 bytes a value): no more CTAs than slots
     const uint64_t grid = std::min<uint64_t>(std::min<uint64_t>(nb, slots), (uint64_t)sms * (uint64_t)std::max(per_sm, 1));
     partition_cta_kernel<<<(unsigned)grid, 32 * kPartWarps, smem, st>>>(A);
   } else {

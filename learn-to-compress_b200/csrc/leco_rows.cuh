@@ -1,13 +1,14 @@
 // leco_rows.cuh -- the row encoder: one thread per row of 32 consecutive values.
 //
-// A block of bs values is handled by R threads (R a power of two, 8 .. 512, R >= bs / 32);
+// A block of bs values is handled by R threads (R >= bs / 32, 8 .. 512: a power of two in the
+// batch engine and for blocks that share a CTA, else as many warps as the rows need);
 // thread t takes values 32t .. 32t+31, its row of shared memory, in every pass.  A row's
 // fields pack into whole 32-bit words (32 fields of l bits are l words) without any sharing
 // between threads, residuals replace the values they came from, and nothing but running
-// maxima and sums stays in registers, so that six CTAs of four warps fit an SM.  A CTA of NT threads encodes NT / R consecutive blocks (an item) and
-// takes one look-back for all of them.  Used by the single-column kernels
-// (leco_encode.cu) and the batch engine (leco_batch_encode.cu); blocks are the
-// reference's images byte for byte.
+// maxima and sums stays in registers, so that six CTAs of four warps fit an SM.  A CTA of NT
+// threads encodes NT / R consecutive blocks (an item) and takes one offset for all of them.
+// Used by the single-column kernels (leco_rows_kernel.cuh) and the batch engine
+// (leco_batch_encode.cu); blocks are the reference's images byte for byte.
 //
 // The reference's fit adds a block's values (and i * value, i * i * value) one after the
 // other in FP64 (lr.h:72-77, polynomial_regression_internals.hpp:129-137).  rows_fit
@@ -33,9 +34,9 @@
 // u64 Delta 6.2K, u64 LeCo 8.8K, with the fit's chains 12.6K; issue slots 45-60 % busy, the
 // rest barriers within the block and the wait for the item's offset).  Against the encoder
 // with one CTA per block that gathered each output chunk field by field, or staged twice:
-// one 4096-value u64 block 82 -> 13 us (host-bound), 1M u32 LeCo in blocks of 1000 34.8 -> 16 us,
-// 30M u32 FOR 130 -> 55 us, 20M u64 Delta in blocks of 2048 176 -> 68 us, 100M u64 LeCo (fits
-// from the fit kernel, leco_encode.cu) 557 -> 450 us.
+// one 4096-value u64 block 82 -> 13 us (host-bound), 1M u32 LeCo in blocks of 1000 34.8 -> 15.4 us,
+// 30M u32 FOR 130 -> 58 us, 20M u64 Delta in blocks of 2048 176 -> 72 us, 100M u64 LeCo (fits
+// from the fit kernel, leco_encode.cu) 557 -> 464 us.
 #pragma once
 #include "leco_encode.cuh"
 
@@ -129,8 +130,8 @@ struct RowGroup {
 
 // Max, min and (OR) or of 32-bit values over the group; `slots`: u64 [2][warps] that no
 // thread still reads (successive reductions alternate between two sets).  (64-bit reductions
-// go by shuffles: as two redux.sync on the halves, the second on a selected operand, nvcc
-// 12.9 returned the registers' earlier contents in one kernel.)
+// go by shuffles: as two redux.sync on the halves, the second on a selected operand, they gave
+// wrong maxima in one kernel, and the cause was not found.)
 template <bool OR, uint32_t RT>
 __device__ __forceinline__ void rg_reduce3(const RowGroup<RT> &g, int32_t &mx, int32_t &mn, uint32_t &ov, uint64_t *slots) {
   if (g.rl() == 32) {
@@ -1226,7 +1227,7 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
 // ---- offsets of a column's items ------------------------------------------------------
 // A single column's items take their byte offsets from a publisher CTA, the first CTA of the
 // column to start (items are numbered in the order in which theirs started): it walks the status
-// words in item order, kPubWindow of them a step, and turns every published total into an
+// words in item order, up to kPubWindow of them a step, and turns every published total into an
 // inclusive prefix once all the items before it have published theirs.  An item publishes
 // its total, packs, and then polls its own word alone.  Waits are bounded: on expiry the error word
 // is set and the item is not written.

@@ -20,10 +20,10 @@ constexpr int rows_min_ctas() {
 }
 
 // One CTA of NT threads per item of NT / R blocks (RT: R, or 0: 32 and less), or with RT
-// kWholeCta of R <= NT threads per block.  A
-// column of one item needs no other; else the CTAs take their roles from a ticket as they
-// start, since CUDA does not promise the order of their indexes: the first is the publisher,
-// the k-th after it takes item k - 1, so whatever an item waits for has started before it.
+// kWholeCta of R <= NT threads per block.  A column of one item needs no other; else the CTAs
+// take their roles from a ticket as they start, since CUDA does not promise the order of their
+// indexes: the first is the publisher, the k-th after it takes item k - 1, so whatever an item
+// waits for has started before it.
 // The ticket is a trip to L2 before the first load (roles by index / by ticket: 100M u64 LeCo
 // 455 / 464 us, 30M u32 FOR 56.7 / 59.4, 20M u64 Delta 67.6 / 71.0; CTAs that stay and ask for
 // their next ticket ahead: 574, 71, 76).
