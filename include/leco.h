@@ -471,11 +471,16 @@ int leco_check(leco_stream_t stream);
  * returns what leco_check reports afterwards: LECO_ERR_TIMEOUT when the bounded
  * wait gave up as designed (*h_result = ~0).  Synchronous; the context stays usable. */
 int leco_test_bounded_wait(uint32_t spin_limit, uint64_t *h_result);
-/* TEST HOOK of the same kind for the column encoder's waits: part 0 runs its publisher on
- * three items of which only the first has published its total (48), part 1 an item's wait
- * for a publisher that never comes.  h_words (4 words): the items' three status words and,
- * for part 1, the wait's result (~0 when it gave up). */
-int leco_test_rows_wait(uint32_t spin_limit, int part, uint64_t *h_words);
+/* TEST HOOKS of the same kind for the column encoder.  leco_test_rows_wait runs its publisher
+ * on three items of which only the first has published its total (48); h_words (4 words): the
+ * items' three status words and the list's counters.  leco_test_encode_order is leco_encode with
+ * the polls after which an item leaves its place to the publisher (0: the default) and, with
+ * `reversed`, the roles given to the CTAs from the last one down, the order in which every item
+ * starts before those that it waits for. */
+int leco_test_rows_wait(uint32_t spin_limit, uint64_t *h_words);
+int leco_test_encode_order(int codec, int dtype, const void *d_values, uint64_t n, uint32_t block_size, int fit_mode,
+                           uint8_t *d_payload, uint64_t payload_cap, uint64_t *d_offsets, void *d_workspace,
+                           uint64_t workspace_bytes, uint32_t item_wait, int reversed, leco_stream_t stream);
 /* Message of the last error on this thread ("" if none). */
 const char *leco_last_error(void);
 /* Library version string. */

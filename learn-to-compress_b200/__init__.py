@@ -114,7 +114,8 @@ SIGNATURES = [
     ("leco_varlen_gather", _I, [_P, _P, _P, _U64, _U64, _P, _U64, _P, _P]),
     ("leco_varlen_sum", _I, [_P, _P, _P, _U64, _U64, _P, _P]),
     ("leco_test_bounded_wait", _I, [_U32, _P]),
-    ("leco_test_rows_wait", _I, [_U32, _I, _P]),
+    ("leco_test_rows_wait", _I, [_U32, _P]),
+    ("leco_test_encode_order", _I, [_I, _I, _P, _U64, _U32, _I, _P, _U64, _P, _P, _U64, _U32, _I, _P]),
     ("leco_check", _I, [_P]),
     ("leco_last_error", ctypes.c_char_p, []),
     ("leco_version", ctypes.c_char_p, []),

@@ -22,7 +22,9 @@ __device__ __forceinline__ void batch_encode_one(const BatchArgs &B, const DevCo
   a.status = B.status + c.item0;
   a.ticket = nullptr;
   a.error = B.error;
-  encode_rows_item<T, CODEC, 0, false>(a, item, c.rows, c.seq != 0, false, smem);
+  a.item_wait = 0;
+  a.reversed = false;
+  encode_rows_item<T, CODEC, 0, false>(a, item, c.rows, c.seq != 0, false, false, smem);
 }
 
 // Persistent encode: one ticket = one item of 256 / rows consecutive blocks of a column

@@ -148,9 +148,9 @@ uint64_t leco_encode_workspace_bytes(int codec, int dtype, uint64_t n, uint32_t 
   return enc_ws(nb, needs_seq_fit(codec, dtype, block_size, fit_mode)).total;
 }
 
-int leco_encode(int codec, int dtype, const void *d_values, uint64_t n, uint32_t block_size, int fit_mode,
-                uint8_t *d_payload, uint64_t payload_cap, uint64_t *d_offsets, leco_dir_entry *d_dir,
-                void *d_workspace, uint64_t workspace_bytes, leco_stream_t stream) {
+static int encode_column(int codec, int dtype, const void *d_values, uint64_t n, uint32_t block_size, int fit_mode,
+                         uint8_t *d_payload, uint64_t payload_cap, uint64_t *d_offsets, leco_dir_entry *d_dir,
+                         void *d_workspace, uint64_t workspace_bytes, uint32_t item_wait, bool reversed, leco_stream_t stream) {
   if (!codec_write_ok(codec, dtype))
     return fail(LECO_ERR_UNSUPPORTED, "leco_encode: codec must be LINEAR, FOR, DELTA, POLY2 or LINEAR_F32 (u32)");
   if (!dtype_ok(dtype)) return fail(LECO_ERR_ARG, "leco_encode: dtype must be LECO_U32 or LECO_U64");
@@ -170,7 +170,7 @@ int leco_encode(int codec, int dtype, const void *d_values, uint64_t n, uint32_t
   if (rc) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   uint8_t *ws = static_cast<uint8_t *>(d_workspace);
-  // status words + ticket; a column that is one item of the row encoder uses neither
+  // status words, ticket and list; a column that is one item of the row encoder uses none of them
   if (nb > 1 || codec == kLegacy) LECO_CUDA(cudaMemsetAsync(ws, 0, w.models_off, st));
   EncodeLaunch L;
   L.values = d_values; L.n = n; L.bs = block_size; L.nb = nb;
@@ -179,6 +179,7 @@ int leco_encode(int codec, int dtype, const void *d_values, uint64_t n, uint32_t
   L.status = reinterpret_cast<uint64_t *>(ws + w.status_off);
   L.ticket = reinterpret_cast<uint32_t *>(ws + w.ticket_off);
   L.error = err;
+  L.item_wait = item_wait; L.reversed = reversed;
   for (int i = 0; i < 10; ++i) L.polyX[i] = 0;
   if (codec == kPoly2) {
     poly2_x_sums(std::min<uint64_t>(n, block_size), L.polyX);
@@ -190,6 +191,20 @@ int leco_encode(int codec, int dtype, const void *d_values, uint64_t n, uint32_t
   if (lrc < 0) return cuda_fail((cudaError_t)-lrc, "leco_encode: launch");
   LECO_CUDA(cudaGetLastError());
   return LECO_OK;
+}
+
+int leco_encode(int codec, int dtype, const void *d_values, uint64_t n, uint32_t block_size, int fit_mode,
+                uint8_t *d_payload, uint64_t payload_cap, uint64_t *d_offsets, leco_dir_entry *d_dir,
+                void *d_workspace, uint64_t workspace_bytes, leco_stream_t stream) {
+  return encode_column(codec, dtype, d_values, n, block_size, fit_mode, d_payload, payload_cap, d_offsets, d_dir, d_workspace,
+                       workspace_bytes, 0, false, stream);
+}
+
+int leco_test_encode_order(int codec, int dtype, const void *d_values, uint64_t n, uint32_t block_size, int fit_mode,
+                           uint8_t *d_payload, uint64_t payload_cap, uint64_t *d_offsets, void *d_workspace,
+                           uint64_t workspace_bytes, uint32_t item_wait, int reversed, leco_stream_t stream) {
+  return encode_column(codec, dtype, d_values, n, block_size, fit_mode, d_payload, payload_cap, d_offsets, nullptr, d_workspace,
+                       workspace_bytes, item_wait, reversed != 0, stream);
 }
 
 static int check_column(const char *fn, int codec, int dtype, const void *payload, const void *offsets, uint32_t bs) {

@@ -271,6 +271,7 @@ int launch_encode(int codec, int s, const EncodeLaunch &L, cudaStream_t st) {
   a.values = L.values; a.n = L.n; a.bs = L.bs; a.nb = L.nb;
   a.payload = L.payload; a.payload_cap = L.payload_cap; a.offsets = L.offsets; a.dir = L.dir;
   a.seq_models = nullptr; a.status = L.status; a.ticket = L.ticket; a.error = L.error;
+  a.item_wait = L.item_wait ? L.item_wait : kItemWait; a.reversed = L.reversed;
   for (int i = 0; i < 10; ++i) a.polyX[i] = L.polyX[i];
   if (codec != kLegacy) {
     const bool ref = L.seq_models != nullptr;
@@ -308,18 +309,12 @@ __global__ void lookback_timeout_probe_kernel(uint64_t *status, uint32_t *error,
     if (threadIdx.x == 0) *result = excl;
   }
 }
-// The row encoder's two waits: the publisher of three items of which the second never
-// publishes its total (part 0), and an item whose word the publisher never reaches (part 1).
-__global__ void __launch_bounds__(128) rows_timeout_probe_kernel(uint64_t *status, uint32_t *error, uint32_t spin_limit, int part,
-                                                                 uint64_t *result) {
+// The row encoder's publisher, of three items of which the second never publishes its total.
+__global__ void __launch_bounds__(128) rows_timeout_probe_kernel(uint64_t *status, uint32_t *error, uint32_t spin_limit) {
   __shared__ __align__(16) uint8_t scratch[256];
-  if (part == 0) {
-    if (threadIdx.x == 0) status[0] = kFlagAgg | 48;
-    __syncthreads();
-    publish_items<128>(status, 3, error, scratch, spin_limit);
-  } else if (threadIdx.x == 0) {
-    *result = await_prefix(status, 1, 16, error, spin_limit);
-  }
+  if (threadIdx.x == 0) status[0] = kFlagAgg | 48;
+  __syncthreads();
+  publish_items<128, true>(status, 3, reinterpret_cast<uint32_t *>(status + 3), error, scratch, spin_limit);
 }
 
 }  // namespace leco
@@ -354,11 +349,11 @@ extern "C" int leco_test_bounded_wait(uint32_t spin_limit, uint64_t *h_result) {
   return rc;
 }
 
-extern "C" int leco_test_rows_wait(uint32_t spin_limit, int part, uint64_t *h_words) {
-  if (part < 0 || part > 1 || !h_words) return leco::record_error(LECO_ERR_ARG, "leco_test_rows_wait: part 0 or 1, four words");
+extern "C" int leco_test_rows_wait(uint32_t spin_limit, uint64_t *h_words) {
+  if (!h_words) return leco::record_error(LECO_ERR_ARG, "leco_test_rows_wait: four words");
   uint64_t words[4] = {0, 0, 0, 0};
   const int rc = run_wait_probe("leco_test_rows_wait", words, [&](uint64_t *w, uint32_t *err) {
-    leco::rows_timeout_probe_kernel<<<1, 128>>>(w, err, spin_limit, part, w + 3);
+    leco::rows_timeout_probe_kernel<<<1, 128>>>(w, err, spin_limit);
   });
   for (int i = 0; i < 4; ++i) h_words[i] = words[i];
   return rc;

@@ -31,8 +31,10 @@ struct EncodeArgs {
   const double *seq_models;  // [nb*3] or null (exact fit in-kernel)
   double polyX[10];          // X sums for full blocks [0..4] and for the tail block [5..9]
   uint64_t *status;          // [nb] look-back words, zeroed
-  uint32_t *ticket;          // zeroed
+  uint32_t *ticket;          // zeroed: [0] the legacy encoder's ticket, [1..3] the row encoder's left items
   uint32_t *error;           // error word
+  uint32_t item_wait;        // row encoder: polls after which an item leaves its place
+  bool reversed;             // row encoder: the last CTA takes the first role (tests)
 };
 
 // Shared-memory layout helper.

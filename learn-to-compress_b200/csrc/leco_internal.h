@@ -23,6 +23,8 @@ struct EncodeLaunch {
   uint64_t *status;
   uint32_t *ticket;
   uint32_t *error;
+  uint32_t item_wait = 0;  // row encoder: polls before an item leaves its place (0: the default)
+  bool reversed = false;   // row encoder: roles from the last CTA down (tests)
 };
 
 struct DecodeLaunch {

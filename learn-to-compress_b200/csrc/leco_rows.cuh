@@ -68,7 +68,7 @@ __host__ __device__ constexpr int rows_sums(int codec) { return codec == kLinear
 // Shared memory of one CTA of nt threads in groups of R; from tab on for the reference's fit
 // in the encoder only (`total` with it, `tab` without).
 struct RowsLayout {
-  uint32_t wtot, red, hdr, model, size, goff, count, tab, base, mask, total;
+  uint32_t wtot, red, hdr, model, size, goff, count, next, tab, base, mask, total;
 };
 __host__ __device__ constexpr RowsLayout rows_layout(uint32_t nt, uint32_t R, uint32_t s, uint32_t ns) {
   RowsLayout L{};
@@ -80,7 +80,8 @@ __host__ __device__ constexpr RowsLayout rows_layout(uint32_t nt, uint32_t R, ui
   L.model = L.hdr;                          // double [groups][4]: read before the header is made
   L.size = o;  o += ng * 8;                 // u64 [groups]
   L.goff = o;  o += ng * 8;                 // u64 [groups]
-  L.count = o; o += 8;                      // u32: groups whose size is known
+  L.count = o; o += 4;                      // u32: groups whose size is known
+  L.next = o;  o += 4;                      // u32: the next item that had left its place
   L.tab = o;   o += ns * nt * 8;            // [ns][nt]: a row's effect (four int16) or its run's (two int32)
   L.base = o;  o += ns * (nt + ng) * 8;     // u64 [ns][groups * (R + 1)]: the rows' approximate starts
   L.mask = o;  o += ns * nw * 8;            // uint2 [ns][warps]: rows to walk, uncertain rows
@@ -1225,23 +1226,43 @@ __device__ __forceinline__ void encode_rows_passes(const EncodeArgs &a, const Ro
 }
 
 // ---- offsets of a column's items ------------------------------------------------------
-// A single column's items take their byte offsets from a publisher CTA, the first CTA of the
-// column to start (items are numbered in the order in which theirs started): it walks the status
+// A single column's items take their byte offsets from a publisher CTA: it walks the status
 // words in item order, up to kPubWindow of them a step, and turns every published total into an
 // inclusive prefix once all the items before it have published theirs.  An item publishes
-// its total, packs, and then polls its own word alone.  Waits are bounded: on expiry the error word
-// is set and the item is not written.
+// its total, packs, and then polls its own word alone.
+// Roles go by blockIdx, the publisher first.  CTAs do start in that order as far as anyone has
+// seen, but CUDA does not promise it, and if an item that has not started were kept from starting
+// by items that wait for it, none would end.  So an item that has polled `item_wait` times leaves
+// its place: it puts itself on a list and ends without its image, so that other CTAs can start,
+// and the publisher encodes the items of the list again when every prefix is out.  (Tickets, taken
+// as the CTAs start, would order them too, but 1500 CTAs asking one word at once wait 6 us for it:
+// 10M u32 Delta values in blocks of 4096 21 us by index, 26 by ticket; 30M u32 FOR 55.1 / 58.3;
+// 100M u64 LeCo 454 / 469; CTAs that stay and ask for their next ticket ahead: 71 and 574.)
+// Leaving and publishing meet in the item's word.  The item counts itself (left[0]), fences,
+// and exchanges its total for the same with kLeft, which fails if the prefix is there; the
+// publisher writes the prefixes, fences, and reads left[0].  Whichever word came first, either the
+// exchange fails or the publisher sees the count; it then waits until all that are counted
+// have gone on or are on the list (left[1]).  All waits are bounded: on the publisher's expiry the
+// error word is set and items may be left unwritten.
 // The items in flight (~900 to 1500) wait for the step, and a step is a read of L2 and two
 // barriers, so its width matters both ways: 24.6M u32 FOR / Delta values, us: windows of 128
 // words 47 / 48, 256 42 / 44, 512 41 / 44, 1024 50 / 51; one warp stepping over 256 words 47 / 50.
+constexpr uint64_t kLeft = 1ull << 61, kSizeMask = kLeft - 1;
+constexpr uint32_t kItemWait = 1u << 16;  // some 40 ms; an item waits for tens of microseconds
+__device__ __forceinline__ uint32_t ld_relaxed32(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
 constexpr uint32_t kPubWindow = 512;
-template <uint32_t NT>  // at most NT threads
-__device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, uint32_t *error, uint8_t *smem,
-                                              uint32_t spin_limit = kSpinLimit) {
+// Returns the head of the list of left items (item + 1; 0: none), the same in every thread.
+template <uint32_t NT, bool FIXED>  // NT threads, or at most NT
+__device__ __forceinline__ uint32_t publish_items(uint64_t *status, uint64_t items, uint32_t *left, uint32_t *error, uint8_t *smem,
+                                                  uint32_t spin_limit = kSpinLimit) {
   constexpr uint32_t NW = NT / 32, kPubWords = kPubWindow / NT;
   uint64_t *wsum = reinterpret_cast<uint64_t *>(smem);                // [2][NW]
   uint32_t *wfirst = reinterpret_cast<uint32_t *>(smem + 2 * NW * 8);  // [2][NW]
-  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5, window = kPubWords * blockDim.x;
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5, nw = FIXED ? NW : blockDim.x >> 5, window = kPubWords * 32 * nw;
   uint64_t run = 0, j = 0;  // inclusive prefix before item j
   uint32_t spins = 0, par = 0;
   while (j < items) {
@@ -1258,7 +1279,7 @@ __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, 
       if ((v[k] >> 62) == 0) first = kPubWords * t + k;
 #pragma unroll
     for (uint32_t k = 0; k < kPubWords; ++k)
-      if (kPubWords * t + k < first) own += v[k] & kValMask;
+      if (kPubWords * t + k < first) own += v[k] & kSizeMask;
     first = __reduce_min_sync(0xffffffffu, first);
     uint64_t incl = own;
 #pragma unroll
@@ -1284,7 +1305,7 @@ __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, 
     for (uint32_t k = 0; k < kPubWords; ++k) {
       const uint32_t place = kPubWords * t + k;
       if (place < n) {
-        before += v[k] & kValMask;
+        before += v[k] & kSizeMask;
         st_relaxed(&status[j + place], kFlagIncl | before);
         if (place == n - 1) {
           last = before;
@@ -1297,7 +1318,7 @@ __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, 
     if (n == 0) {
       if (++spins > spin_limit) {
         if (t == 0) atomicOr(error, kErrTimeout);
-        return;
+        return 0;
       }
       __nanosleep(32);
     } else {
@@ -1308,29 +1329,64 @@ __device__ __forceinline__ void publish_items(uint64_t *status, uint64_t items, 
     j += n;
     par ^= 1;
   }
-}
-// One warp: the item's exclusive prefix, once the publisher has replaced its total by the
-// inclusive prefix; ~0 when the wait gave up.
-__device__ __forceinline__ uint64_t await_prefix(const uint64_t *status, uint64_t item, uint64_t total, uint32_t *error,
-                                                 uint32_t spin_limit = kSpinLimit) {
-  uint32_t spins = 0;
-  for (;;) {
-    const uint64_t v = ld_relaxed(&status[item]);
-    if ((v >> 62) == 2) return (v & kValMask) - total;
-    if (++spins > spin_limit) {
-      atomicOr(error, kErrTimeout);
-      return ~0ull;
+  __threadfence();
+  __syncthreads();
+  uint32_t *head = reinterpret_cast<uint32_t *>(smem);
+  if (t == 0) {
+    __threadfence();
+    uint32_t h = 0;
+    if (ld_relaxed32(left)) {
+      // (what is done is read before what is counted: equal, they are all done)
+      for (spins = 0;;) {
+        const uint32_t done = ld_relaxed32(left + 1);
+        __threadfence();
+        if (done == ld_relaxed32(left)) {
+          h = ld_relaxed32(left + 2);
+          break;
+        }
+        if (++spins > spin_limit) {
+          atomicOr(error, kErrTimeout);
+          break;
+        }
+        __nanosleep(64);
+      }
     }
+    *head = h;
+  }
+  __syncthreads();
+  const uint32_t h = *head;
+  __syncthreads();
+  return h;
+}
+// One lane: the item's exclusive prefix, once the publisher has replaced its total by the
+// inclusive prefix; ~0 when the item has left its place (link: the word of the list's next).
+__device__ __forceinline__ uint64_t await_prefix(uint64_t *status, uint64_t item, uint64_t total, uint32_t *left, uint64_t *link,
+                                                 uint32_t wait) {
+  for (uint32_t polls = 0;; ++polls) {
+    const uint64_t v = ld_relaxed(&status[item]);
+    if ((v >> 62) == 2) return (v & kSizeMask) - total;
+    if (polls >= wait) break;
     __nanosleep(64);
   }
+  atomicAdd(left, 1u);
+  __threadfence();
+  const unsigned long long mine = kFlagAgg | total;
+  const uint64_t was = atomicCAS(reinterpret_cast<unsigned long long *>(&status[item]), mine, mine | kLeft);
+  if (was == mine) {
+    *link = atomicExch(left + 2, (uint32_t)item + 1u);
+    __threadfence();
+  }
+  atomicAdd(left + 1, 1u);
+  return was == mine ? ~0ull : (was & kSizeMask) - total;
 }
 
 // ---- one item: the NT / R blocks from item * (NT / R) on ------------------------------
 // Every thread of the CTA calls it.  ref: the reference's sequential fit (else the exact
 // moments).  a.status has one word per item; PUB: a publisher CTA turns them into prefixes,
-// else the item looks back itself (alone: the column's only item).  smem: rows_layout's bytes, 256-byte aligned.
+// else the item looks back itself (alone: the column's only item; again: an item that had left
+// its place).  smem: rows_layout's bytes, 256-byte aligned.
 template <typename T, int CODEC, uint32_t RT, bool PUB>
-__device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t item, uint32_t Rd, bool ref, bool alone,
+__device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t item, uint32_t Rd, bool ref, bool alone, bool again,
                                                  uint8_t *smem) {
   constexpr uint32_t S = sizeof(T), TB = 8 * S;
   const RowGroup<RT> g(Rd);
@@ -1355,7 +1411,7 @@ __device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t i
   // do not: the last rows' warp then held up all others, and both forms of the passes in use at
   // once cost more than the masks of the one -- 60M u64, exact fit, blocks of 3000: LeCo 439 us,
   // 390 so; poly2 671, 518.  FOR and Delta are faster with both.)
-  uint64_t *status = alone ? nullptr : a.status + item;
+  uint64_t *status = alone || again ? nullptr : a.status + item;
   constexpr bool kModel = CODEC == kLinear || CODEC == kPoly2;
   if (__all_sync(0xffffffffu, kModel ? len == 32 * R : P.cnt == 32)) encode_rows_passes<T, CODEC, true>(a, P, ref, sb, smem, L, b, C, status);
   else encode_rows_passes<T, CODEC, false>(a, P, ref, sb, smem, L, b, C, status);
@@ -1403,7 +1459,7 @@ __device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t i
     __syncwarp();
     uint64_t excl;
     if (PUB) {
-      excl = g.lane == 0 && !alone ? await_prefix(a.status, item, total, a.error) : 0;
+      excl = g.lane == 0 && !alone ? await_prefix(a.status, item, total, a.ticket + 1, a.offsets + item * NB, a.item_wait) : 0;
       excl = __shfl_sync(0xffffffffu, (unsigned long long)excl, 0);
     } else {
       excl = lookback_excl(a.status, item, a.error);
@@ -1413,7 +1469,7 @@ __device__ __forceinline__ void encode_rows_item(const EncodeArgs &a, uint64_t i
   }
   __syncthreads();
   const uint64_t goff = goffs[g.gi];
-  if (!len || goff == ~0ull) return;  // (look-back gave up: error word set)
+  if (!len || goff == ~0ull) return;  // (the item has left its place, or the look-back gave up: error word set)
   if (goff + size + LECO_PAYLOAD_SLACK > a.payload_cap) {  // never write past the buffer
     if (g.rank == 0) atomicOr(a.error, kErrCapacity);
     return;

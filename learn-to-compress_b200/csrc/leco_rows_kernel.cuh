@@ -20,27 +20,33 @@ constexpr int rows_min_ctas() {
 }
 
 // One CTA of NT threads per item of NT / R blocks (RT: R, or 0: 32 and less), or with RT
-// kWholeCta of R <= NT threads per block.  A column of one item needs no other; else the CTAs
-// take their roles from a ticket as they start, since CUDA does not promise the order of their
-// indexes: the first is the publisher, the k-th after it takes item k - 1, so whatever an item
-// waits for has started before it.
-// The ticket is a trip to L2 before the first load (roles by index / by ticket: 100M u64 LeCo
-// 455 / 464 us, 30M u32 FOR 56.7 / 59.4, 20M u64 Delta 67.6 / 71.0; CTAs that stay and ask for
-// their next ticket ahead: 574, 71, 76).
+// kWholeCta of R <= NT threads per block.  A column of one item needs no other; else CTA 0 is the
+// publisher and CTA i + 1 takes item i (see the offsets in leco_rows.cuh).
 template <typename T, int CODEC, int NT, uint32_t RT>
 __global__ void __launch_bounds__(rows_max_threads<T, CODEC, NT>(), rows_min_ctas<T, CODEC, NT>())
     encode_rows_kernel(EncodeArgs a, uint32_t R, uint32_t items, bool ref) {
   extern __shared__ __align__(256) uint8_t smem_raw[];
-  uint32_t role = 1;
-  if (items > 1) {
-    // (the place of the groups' offsets, which are written after further barriers)
-    uint32_t *ticket = reinterpret_cast<uint32_t *>(smem_raw + rows_layout(RT == kWholeCta ? R : NT, RT && RT != kWholeCta ? RT : R, sizeof(T), 0).goff);
-    if (threadIdx.x == 0) *ticket = atomicAdd(a.ticket, 1u);
-    __syncthreads();
-    role = *ticket;
+  const bool alone = items == 1;
+  const uint32_t role = a.reversed ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const bool again = !alone && role == 0;
+  uint32_t item = alone ? 0 : role - 1;
+  if (again) {
+    const uint32_t head = publish_items<NT, RT != kWholeCta>(a.status, items, a.ticket + 1, a.error, smem_raw);
+    if (!head) return;
+    item = head - 1;
   }
-  if (role == 0) publish_items<NT>(a.status, items, a.error, smem_raw);
-  else encode_rows_item<T, CODEC, RT, true>(a, role - 1, R, ref, items == 1, smem_raw);
+  for (;;) {
+    // the list goes on in the place of the item's first offset, which the item writes at its end
+    uint32_t *next =
+        reinterpret_cast<uint32_t *>(smem_raw + rows_layout(RT == kWholeCta ? R : NT, RT && RT != kWholeCta ? RT : R, sizeof(T), 0).next);
+    if (again && threadIdx.x == 0) *next = (uint32_t)ld_relaxed(a.offsets + (uint64_t)item * ((RT == kWholeCta ? R : NT) / R));
+    encode_rows_item<T, CODEC, RT, true>(a, item, R, ref, alone, again, smem_raw);
+    if (!again) return;
+    __syncthreads();
+    if (!*next) return;
+    item = *next - 1;
+    __syncthreads();
+  }
 }
 
 template <typename T, int CODEC, int NT, uint32_t RT>
