@@ -5,7 +5,7 @@
 // thread t takes values 32t .. 32t+31, its row of shared memory, in every pass.  A row's
 // fields pack into whole 32-bit words (32 fields of l bits are l words) without any sharing
 // between threads, residuals replace the values they came from, and nothing but running
-// maxima and sums stays in registers, so that six CTAs of four warps fit an SM.  A CTA of NT
+// maxima and sums stays in registers, so that six CTAs of four warps (u64) fit an SM.  A CTA of NT
 // threads encodes NT / R consecutive blocks (an item) and takes one offset for all of them.
 // Used by the single-column kernels (leco_rows_kernel.cuh) and the batch engine
 // (leco_batch_encode.cu); blocks are the reference's images byte for byte.
@@ -30,13 +30,13 @@
 // from the exact sum before it, unless that sum is one of the starts tried.  When the total
 // of a sum is below 2^53 every partial sum is an exact integer and the scan's total is it.
 //
-// What bounds it: instructions (4096-value blocks, warp instructions per block: u32 FOR 3.8K,
-// u64 Delta 6.2K, u64 LeCo 8.8K, with the fit's chains 12.6K; issue slots 45-60 % busy, the
-// rest barriers within the block and the wait for the item's offset).  Against the encoder
+// What bounds it: instructions (4096-value blocks, warp instructions per block: u32 FOR 4.0K,
+// u64 Delta 6.3K, u64 LeCo with the fit's chains 13K; issue slots 48-56 % busy, the rest
+// barriers within the block and the wait for the item's offset).  Against the encoder
 // with one CTA per block that gathered each output chunk field by field, or staged twice:
 // one 4096-value u64 block 82 -> 13 us (host-bound), 1M u32 LeCo in blocks of 1000 34.8 -> 15.4 us,
-// 30M u32 FOR 130 -> 58 us, 20M u64 Delta in blocks of 2048 176 -> 72 us, 100M u64 LeCo (fits
-// from the fit kernel, leco_encode.cu) 557 -> 464 us.
+// 30M u32 FOR 130 -> 57 us, 20M u64 Delta in blocks of 2048 176 -> 66 us, 100M u64 LeCo (fits
+// from the fit kernel, leco_encode.cu) 557 -> 460 us.
 #pragma once
 #include "leco_encode.cuh"
 
